@@ -144,6 +144,22 @@ def pilot_depth(layer_sizes: list[int], gens: int, work: int = PILOT_WORK) -> in
     return len(layer_sizes)
 
 
+def runs_coset_layers(graph: GraphDefinition, device: int = 0) -> bool:
+    """Whether the default plan of `graph` runs a whole search in coset-word
+    layers (the Lehmer bitmap of distinct labels, up to 14 symbols and 32
+    generators)."""
+    if graph.action["kind"] != "permutation" or len(graph.start) > 14 or graph.generator_count > 32:
+        return False
+    from .engine import NativeGraph
+    from . import native
+    try:
+        with NativeGraph(graph, device) as eng:
+            info = eng.plan()
+    except native.NativeError:
+        return False
+    return info["visited"] == "bitmap" and info["rank_components"] == 1 and len(set(graph.start)) == len(graph.start)
+
+
 def _run_pilot(graph, plan, device, max_layers, max_seconds, info=None):
     from .engine import NativeGraph
     from . import native
@@ -165,7 +181,8 @@ def _trials(graph, plans, device, depth, per_trial, first, started, budget_secon
         if time.perf_counter() - started > budget_seconds:
             break
         r = _run_pilot(graph, plan, device, depth, per_trial)
-        ok = r is not None and r.layer_sizes[:depth] == first.layer_sizes[:depth] and len(r.layer_sizes) >= depth
+        want = first.layer_sizes[:depth]
+        ok = r is not None and r.layer_sizes[:depth] == want and len(r.layer_sizes) >= len(want)
         trials.append({"plan": plan, "seconds": r.device_seconds if ok else None})
     return trials
 
@@ -190,11 +207,20 @@ def choose_profile(graph: GraphDefinition, device: int = 0, *, budget_seconds: f
     started = time.perf_counter()
     plans = candidate_plans(graph)
     per_trial = max(1.0, budget_seconds / (2 * len(plans)))
+    # Coset-word layers run whole searches only, and a prefix of list layers
+    # says nothing about them (S13 LRX: 35 ms, the fastest list layers 144 ms).
+    # Where a whole search is as cheap as a pilot every candidate runs one; the
+    # larger ones keep the default.
+    whole = runs_coset_layers(graph, device)
+    if whole and _state_bound(graph) * graph.generator_count > PILOT_WORK:
+        return {"plan": dict(DEFAULT), "source": "size", "trials": []}
+    if whole:
+        per_trial = None
     # The default plan's pilot fixes the layer prefix every candidate expands.
     first = _run_pilot(graph, plans[0], device, None, per_trial)
     if first is None:
         return {"plan": dict(DEFAULT), "source": "pilot", "trials": []}
-    depth = pilot_depth(first.layer_sizes, graph.generator_count)
+    depth = None if whole else pilot_depth(first.layer_sizes, graph.generator_count)
     trials = _trials(graph, plans, device, depth, per_trial, first, started, budget_seconds)
     choice = pick(trials)
     # Stage 2: the shapes of the kept path, with the same rule.
@@ -207,9 +233,9 @@ def choose_profile(graph: GraphDefinition, device: int = 0, *, budget_seconds: f
             trials += shape_trials
     if use_cache:
         entries = load_cache(path)
-        entries[key] = {"plan": choice, "trials": trials, "pilot_layers": depth}
+        entries[key] = {"plan": choice, "trials": trials, "pilot_layers": depth or len(first.layer_sizes)}
         store_cache(path, entries)
-    return {"plan": choice, "source": "pilot", "trials": trials, "pilot_layers": depth}
+    return {"plan": choice, "source": "pilot", "trials": trials, "pilot_layers": depth or len(first.layer_sizes)}
 
 
 SWEEP_SAMPLE = 64                  # instances a sweep pilot runs

@@ -115,6 +115,10 @@ int Graph::write_checkpoint(const char* path) {
   if (!checkpointable(visit)) return MGBFS2_UNSUPPORTED;
   MG_CHECK(cudaSetDevice(device));
   MG_CHECK(cudaStreamSynchronize(stream));
+  if (coset_ran) {
+    // A complete search in coset-word layers left no Lehmer bitmap.
+    if (int rc = run_lists(nullptr, nullptr, nullptr, nullptr)) return rc;
+  }
   if (front_grouped) {
     if (int rc = gather_front(last_count)) return rc;
   }

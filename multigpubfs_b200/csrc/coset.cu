@@ -1,0 +1,804 @@
+// Coset-word layers (see coset.h for the coordinates): tables, the persistent
+// wave kernel, the read-out of the deepest layer, and their host side.
+#include "coset.h"
+
+#include <algorithm>
+#include <cstring>
+
+#define MG_CHECK_COSET(expr)                       \
+  do {                                             \
+    cudaError_t _e = (expr);                       \
+    if (_e != cudaSuccess) return cuda_status(_e); \
+  } while (0)
+
+namespace mgbfs2 {
+namespace {
+
+constexpr uint32_t kSlots = 7, kSlotPerms = 5040;
+constexpr uint32_t kCosetBlock = 256, kCosetWarps = kCosetBlock / 32;
+constexpr uint32_t kMaxUnits = 8;  // units (128 nodes) of a work item
+
+struct CosetInst {
+  uint32_t m, gens, rows, inverse_closed;
+  uint32_t same_layer;  // some generator is an even permutation: a layer may have edges inside it
+  uint32_t perm_off;    // first byte of gens x 16 position images
+  unsigned long long row_off, desc_off;  // first row in the buffers and flags; first descriptor
+};
+
+struct CosetCtl {
+  uint32_t arrived, error, steps, pad;
+  unsigned long long collected;  // states of the deepest layer written out
+};
+
+// What the host reads of a wave of one job: pinned memory that the kernel
+// writes at its end, so that the launch and one synchronisation are the whole
+// read-back.  Layers past kReportLayers are copied from the tables.
+constexpr uint32_t kReportLayers = 256;
+struct CosetReport {
+  uint32_t steps, error, previous_count, pad;
+  unsigned long long collected;
+  unsigned long long counts[kReportLayers], stamps[kReportLayers];
+  unsigned long long previous[kCosetSmall], deepest[kCosetSmall];
+};
+
+struct CosetParams {
+  const CosetInst* inst;
+  const uint32_t* item_prefix;  // count + 1: exclusive prefix of the jobs' work items
+  const uint8_t* perms;
+  uint32_t count, units;        // jobs; units per item (a power of two)
+  uint32_t stride, max_steps;   // layer-table columns; last step that may run
+  unsigned long long* counts;   // count x stride layer sizes
+  uint32_t* active;             // stride: layer d of any job is not empty
+  unsigned long long* stamps;   // stride: globaltimer at the start of step d
+  uint8_t* used;                // slot permutations that some row needs
+  uint16_t* table;              // slot permutation x node -> node | flips << 13
+  unsigned long long* desc;     // row x generator -> parent row | slot permutation << 32 | outer flips << 48
+  unsigned long long* flags[2]; // per row: byte p = part p of the buffer's row is not zero
+  void* buf[2];
+  void* visited;                // jobs that are not inverse-closed
+  uint32_t* small_count;        // stride: states kept by step d (wave of one job)
+  unsigned long long* small;    // 2 x kCosetSmall state indices, by step parity
+  CosetReport* report;          // wave of one job: written at the end, else null
+  unsigned long long* front;    // with report: states of the deepest layer, as far as front_cap
+  unsigned long long front_cap, start;  // start: the start's codes, 4 bits each
+  uint32_t n, pad;
+  unsigned long long descs;     // total descriptors
+  CosetCtl* ctl;
+};
+
+__host__ __device__ __forceinline__ void pair_of(uint32_t c, uint32_t* i, uint32_t* j) {
+  uint32_t b = 1;
+  while (b * (b + 1) / 2 <= c) ++b;
+  *j = b;
+  *i = c - b * (b - 1) / 2;
+}
+
+__host__ __device__ __forceinline__ uint32_t bits_below(uint32_t mask, uint32_t p) {
+  const uint32_t x = mask & ((1u << p) - 1u);
+#ifdef __CUDA_ARCH__
+  return __popc(x);
+#else
+  return static_cast<uint32_t>(__builtin_popcount(x));
+#endif
+}
+
+// The i-th position not in `used`.
+__host__ __device__ __forceinline__ uint32_t nth_free(uint32_t used, uint32_t i) {
+  uint32_t p = 0;
+  for (;; ++p)
+    if (!((used >> p) & 1u) && i-- == 0) return p;
+}
+
+// Positions of the outer labels 7 .. m-1 of a row, each pair's lower position
+// first, and the mask of all of them.
+__host__ __device__ __forceinline__ uint32_t row_positions(uint32_t m, uint32_t row, uint8_t* pos) {
+  const uint32_t outer = m - kSlots, pairs = outer / 2;
+  uint32_t digit[4];
+  if (outer & 1) {
+    digit[pairs] = row % 8;
+    row /= 8;
+  }
+  for (uint32_t t = pairs; t-- > 0;) {
+    const uint32_t c = m - 2 * t, radix = c * (c - 1) / 2;
+    digit[t] = row % radix;
+    row /= radix;
+  }
+  uint32_t used = 0;
+  for (uint32_t t = 0; t < pairs; ++t) {
+    uint32_t i, j;
+    pair_of(digit[t], &i, &j);
+    const uint32_t a = nth_free(used, i), b = nth_free(used, j);
+    pos[2 * t] = static_cast<uint8_t>(a);
+    pos[2 * t + 1] = static_cast<uint8_t>(b);
+    used |= (1u << a) | (1u << b);
+  }
+  if (outer & 1) {
+    const uint32_t a = nth_free(used, digit[pairs]);
+    pos[outer - 1] = static_cast<uint8_t>(a);
+    used |= 1u << a;
+  }
+  return used;
+}
+
+// The row whose outer labels sit at `pos` (pairs in either order); *flips
+// gets bit t for every pair whose first label sits at the higher position.
+__host__ __device__ __forceinline__ uint32_t row_rank(uint32_t m, const uint8_t* pos, uint32_t* flips,
+                                                      uint32_t* mask) {
+  const uint32_t outer = m - kSlots, pairs = outer / 2;
+  uint32_t used = 0, row = 0, f = 0;
+  for (uint32_t t = 0; t < pairs; ++t) {
+    uint32_t a = pos[2 * t], b = pos[2 * t + 1];
+    if (a > b) {
+      f |= 1u << t;
+      const uint32_t s = a;
+      a = b;
+      b = s;
+    }
+    const uint32_t i = a - bits_below(used, a), j = b - bits_below(used, b), c = m - 2 * t;
+    row = row * (c * (c - 1) / 2) + j * (j - 1) / 2 + i;
+    used |= (1u << a) | (1u << b);
+  }
+  if (outer & 1) {
+    const uint32_t a = pos[outer - 1];
+    row = row * 8 + a - bits_below(used, a);
+    used |= 1u << a;
+  }
+  *flips = f;
+  *mask = used;
+  return row;
+}
+
+__host__ __device__ __forceinline__ uint32_t rows_of(uint32_t m) {
+  const uint32_t outer = m - kSlots;
+  uint32_t r = outer & 1 ? 8 : 1;
+  for (uint32_t t = 0; t < outer / 2; ++t) r *= (m - 2 * t) * (m - 2 * t - 1) / 2;
+  return r;
+}
+
+// Slots of a node's inner labels, four bits a label, each pair's lower slot
+// first.
+constexpr uint32_t packed_slots(uint32_t x) {
+  const uint32_t digit[3] = {x / 30, x / 3 % 10, x % 3};
+  uint32_t free_slots[kSlots] = {0, 1, 2, 3, 4, 5, 6}, left = kSlots, out = 0;
+  for (uint32_t t = 0; t < 3; ++t) {
+    uint32_t j = 1;
+    while (j * (j + 1) / 2 <= digit[t]) ++j;
+    const uint32_t i = digit[t] - j * (j - 1) / 2;
+    out |= (free_slots[i] | (free_slots[j] << 4)) << (8 * t);
+    uint32_t kept = 0;
+    for (uint32_t k = 0; k < left; ++k)
+      if (k != i && k != j) free_slots[kept++] = free_slots[k];
+    left = kept;
+  }
+  return out | (free_slots[0] << 24);
+}
+struct NodeSlots {
+  uint32_t at[kCosetNodes];
+};
+constexpr NodeSlots all_node_slots() {
+  NodeSlots s{};
+  for (uint32_t x = 0; x < kCosetNodes; ++x) s.at[x] = packed_slots(x);
+  return s;
+}
+__device__ const NodeSlots kNodeSlots = all_node_slots();
+
+// Decoding: the words (4 bits per position, the start's codes) of a row's
+// states share the outer labels in canonical order; an outer or inner flip
+// XORs one pair's two positions.
+struct RowDecode {
+  unsigned long long base, flip[3];
+  uint32_t slots;  // position of each slot, four bits a slot
+};
+
+__device__ __forceinline__ unsigned long long code_of(unsigned long long start, uint32_t label) {
+  return (start >> (4 * label)) & 15ull;
+}
+
+__device__ RowDecode decode_row(uint32_t m, uint32_t row, unsigned long long start) {
+  uint8_t pos[7];
+  const uint32_t used = row_positions(m, row, pos), outer = m - kSlots;
+  RowDecode r{};
+  for (uint32_t l = 0; l < outer; ++l) r.base |= code_of(start, kSlots + l) << (4 * pos[l]);
+#pragma unroll
+  for (uint32_t t = 0; t < 3; ++t)
+    if (t < outer / 2) {
+      const unsigned long long x = code_of(start, kSlots + 2 * t) ^ code_of(start, kSlots + 2 * t + 1);
+      r.flip[t] = (x << (4 * pos[2 * t])) | (x << (4 * pos[2 * t + 1]));
+    }
+  uint32_t s = 0;
+  for (uint32_t at = 0; at < m; ++at)
+    if (!((used >> at) & 1u)) r.slots |= at << (4 * s++);
+  return r;
+}
+
+// The state of bit `bit` of a node's word.
+template <bool WIDE>
+__device__ __forceinline__ unsigned long long decode_state(const RowDecode& r, uint32_t node, uint32_t bit,
+                                                           unsigned long long start, unsigned long long keep) {
+  const uint32_t slots = kNodeSlots.at[node];
+  const uint32_t inner = WIDE ? bit >> 3 : bit >> 2, outer = WIDE ? bit & 7u : bit & 3u;
+  unsigned long long w = r.base;
+#pragma unroll
+  for (uint32_t t = 0; t < 3; ++t) {
+    const uint32_t a = (r.slots >> (4 * ((slots >> (8 * t)) & 15u))) & 15u;
+    const uint32_t b = (r.slots >> (4 * ((slots >> (8 * t + 4)) & 15u))) & 15u;
+    const bool flip = (inner >> t) & 1u;
+    w |= code_of(start, 2 * t) << (4 * (flip ? b : a));
+    w |= code_of(start, 2 * t + 1) << (4 * (flip ? a : b));
+    if ((outer >> t) & 1u) w ^= r.flip[t];
+  }
+  w |= code_of(start, 6) << (4 * ((r.slots >> (4 * ((slots >> 24) & 15u))) & 15u));
+  return w & keep;
+}
+
+// Grid barrier of the cooperative launch: `epoch` counts the barriers passed
+// (the arrival counter only grows).  Bounded like grid_barrier (device.cuh):
+// after kBarrierWaitNs it raises ERR_WAIT_LIMIT and every block ends.
+__device__ __forceinline__ bool coset_barrier(const CosetParams& p, uint32_t* epoch) {
+  __shared__ int ok;
+  __syncthreads();
+  ++*epoch;
+  if (threadIdx.x == 0) {
+    ok = 1;
+    const uint32_t all = *epoch * gridDim.x;
+    uint32_t now;
+    __threadfence();
+    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(now) : "l"(&p.ctl->arrived) : "memory");
+    ++now;
+    const unsigned long long started = global_ns();
+    for (uint32_t polls = 0; static_cast<int32_t>(now - all) < 0; ++polls) {
+      if (polls >= kBarrierPolls || ((polls & 1023u) == 1023u && global_ns() - started > kBarrierWaitNs)) {
+        raise_error(&p.ctl->error, ERR_WAIT_LIMIT);
+        ok = 0;
+        break;
+      }
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&p.ctl->arrived) : "memory");
+    }
+  }
+  __syncthreads();
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+  return ok != 0;
+}
+
+// Descriptors of every (row, generator), the slot permutations they need, and
+// the start states.  The parent of a state under g has the label of position p
+// at position g[p].
+template <typename W>
+__device__ void coset_setup(const CosetParams& p) {
+  const unsigned long long step = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
+  const unsigned long long thread = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x;
+  for (unsigned long long t = thread; t < p.descs; t += step) {
+    uint32_t lo = 0, hi = p.count;
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) / 2;
+      if (p.inst[mid].desc_off <= t) lo = mid;
+      else hi = mid;
+    }
+    const CosetInst in = p.inst[lo];
+    const uint32_t local = static_cast<uint32_t>(t - in.desc_off), row = local / in.gens, g = local % in.gens;
+    const uint8_t* perm = p.perms + in.perm_off + 16 * g;
+    uint8_t pos[7], image[7];
+    const uint32_t used = row_positions(in.m, row, pos);
+    for (uint32_t l = 0; l < in.m - kSlots; ++l) image[l] = perm[pos[l]];
+    uint32_t flips, mask;
+    const uint32_t parent = row_rank(in.m, image, &flips, &mask);
+    // Slot a of the row goes to slot tau[a] of the parent row.
+    uint32_t code = 0, seen = 0, at = 0;
+    for (uint32_t a = 0; a < kSlots; ++a, ++at) {
+      while ((used >> at) & 1u) ++at;
+      const uint32_t image_at = perm[at], tau = image_at - bits_below(mask, image_at);
+      code = code * (kSlots - a) + tau - bits_below(seen, tau);
+      seen |= 1u << tau;
+    }
+    p.used[code] = 1;
+    p.desc[t] = parent | (static_cast<unsigned long long>(code) << 32) | (static_cast<unsigned long long>(flips) << 48);
+  }
+  for (unsigned long long i = thread; i < p.count; i += step) {
+    const CosetInst in = p.inst[i];
+    // The identity: label l at position l, hence node 0 and no flips.
+    uint8_t pos[7];
+    for (uint32_t l = 0; l < kSlots; ++l) pos[l] = static_cast<uint8_t>(kSlots + l);
+    uint32_t f, mask;
+    const unsigned long long row = in.row_off + row_rank(in.m, pos, &f, &mask), w = row * kCosetStride;
+    static_cast<W*>(p.buf[0])[w] = 1;
+    if (!in.inverse_closed) static_cast<W*>(p.visited)[w] = 1;
+    p.flags[0][row] = 1;
+    p.counts[i * p.stride] = 1;
+  }
+  if (thread == 0) p.active[0] = 1;
+}
+
+// The table rows of the slot permutations that some row needs: the image of
+// every node and its inner flips.  One warp takes a permutation.
+__device__ void coset_table(const CosetParams& p) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t warps = gridDim.x * kCosetWarps, warp = blockIdx.x * kCosetWarps + (threadIdx.x >> 5);
+  for (uint32_t base = 0; base * warps + warp < kSlotPerms; base += 32) {
+    const uint32_t mine = (base + lane) * warps + warp;
+    uint32_t found = __ballot_sync(kFullMask, mine < kSlotPerms && __ldcg(p.used + mine));
+    for (; found; found &= found - 1) {
+      const uint32_t perm = (base + __ffs(static_cast<int>(found)) - 1) * warps + warp;
+      // tau, four bits a slot, from its Lehmer code.
+      uint32_t code = perm, digits = 0, tau = 0, seen = 0;
+#pragma unroll
+      for (uint32_t a = kSlots; a-- > 0;) {
+        digits |= (code % (kSlots - a)) << (4 * a);
+        code /= kSlots - a;
+      }
+      for (uint32_t a = 0; a < kSlots; ++a) {
+        const uint32_t to = nth_free(seen, (digits >> (4 * a)) & 15u);
+        tau |= to << (4 * a);
+        seen |= 1u << to;
+      }
+      for (uint32_t x = lane; x < kCosetStride; x += 32) {
+        uint32_t out = x;  // words past the nodes stay zero and map to themselves
+        if (x < kCosetNodes) {
+          const uint32_t slots = kNodeSlots.at[x];
+          uint32_t used = 0, to = 0, flips = 0;
+#pragma unroll
+          for (uint32_t t = 0; t < 3; ++t) {
+            const uint32_t a = (tau >> (4 * ((slots >> (8 * t)) & 15u))) & 15u;
+            const uint32_t b = (tau >> (4 * ((slots >> (8 * t + 4)) & 15u))) & 15u;
+            const uint32_t lo = min(a, b), hi = max(a, b), c = 7 - 2 * t;
+            const uint32_t i = lo - bits_below(used, lo), j = hi - bits_below(used, hi);
+            flips |= (a > b ? 1u : 0u) << t;
+            to = to * (c * (c - 1) / 2) + j * (j - 1) / 2 + i;
+            used |= (1u << a) | (1u << b);
+          }
+          out = to | (flips << 13);
+        }
+        p.table[perm * kCosetStride + x] = static_cast<uint16_t>(out);
+      }
+    }
+  }
+}
+
+// Word with its bit index XORed: inner flips r (per lane), outer flips q (uniform).
+__device__ __forceinline__ uint32_t flip_inner(uint32_t w, uint32_t r) {
+  w = __byte_perm(w, 0u, 0x3210u ^ ((r >> 1) * 0x1111u));
+  const uint32_t s = ((w & 0x0f0f0f0fu) << 4) | ((w >> 4) & 0x0f0f0f0fu);
+  return r & 1u ? s : w;
+}
+__device__ __forceinline__ unsigned long long flip_inner(unsigned long long w, uint32_t r) {
+  const uint32_t lo = static_cast<uint32_t>(w), hi = static_cast<uint32_t>(w >> 32), x = r * 0x1111u;
+  return (static_cast<unsigned long long>(__byte_perm(lo, hi, 0x7654u ^ x)) << 32) | __byte_perm(lo, hi, 0x3210u ^ x);
+}
+__device__ __forceinline__ uint32_t swap_bits(uint32_t w, uint32_t mask, int by) {
+  return ((w & mask) << by) | ((w >> by) & mask);
+}
+__device__ __forceinline__ uint32_t flip_outer(uint32_t w, uint32_t q) {
+  if (q & 1u) w = swap_bits(w, 0x55555555u, 1);
+  if (q & 2u) w = swap_bits(w, 0x33333333u, 2);
+  return w;
+}
+__device__ __forceinline__ unsigned long long flip_outer(unsigned long long w, uint32_t q) {
+  uint32_t lo = static_cast<uint32_t>(w), hi = static_cast<uint32_t>(w >> 32);
+  if (q & 1u) lo = swap_bits(lo, 0x55555555u, 1), hi = swap_bits(hi, 0x55555555u, 1);
+  if (q & 2u) lo = swap_bits(lo, 0x33333333u, 2), hi = swap_bits(hi, 0x33333333u, 2);
+  if (q & 4u) lo = swap_bits(lo, 0x0f0f0f0fu, 4), hi = swap_bits(hi, 0x0f0f0f0fu, 4);
+  return (static_cast<unsigned long long>(hi) << 32) | lo;
+}
+__device__ __forceinline__ uint32_t popcount(uint32_t w) { return __popc(w); }
+__device__ __forceinline__ uint32_t popcount(unsigned long long w) { return __popcll(w); }
+
+template <typename W>
+__device__ __forceinline__ uint32_t lowest_bit(W b) {
+  return (sizeof(W) == 8 ? __ffsll(static_cast<long long>(b)) : __ffs(static_cast<int>(b))) - 1;
+}
+
+// The end of a wave of one job whose step d found nothing: the states of layer
+// d as packed words, in any order, and block 0 writes the report.
+template <typename W>
+__device__ void coset_finish(const CosetParams& p, const CosetInst& in, uint32_t d, bool exhausted) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t warps = gridDim.x * kCosetWarps, warp = blockIdx.x * kCosetWarps + (threadIdx.x >> 5);
+  constexpr bool kWide = sizeof(W) == 8;
+  CosetReport* r = p.report;
+  const unsigned long long keep = (1ull << (4 * p.n)) - 1ull;  // embedded: positions from n up are not written
+  // A layer that `front` does not hold is left to coset_collect.
+  if (exhausted && __ldcg(p.counts + d) <= p.front_cap) {
+    const W* buf = static_cast<const W*>(p.buf[d & 1u]);
+    const unsigned long long* flags = p.flags[d & 1u];
+    for (uint32_t row0 = warp * 32u; row0 < in.rows; row0 += warps * 32u) {
+      const uint32_t row_l = row0 + lane;
+      for (uint32_t m = __ballot_sync(kFullMask, row_l < in.rows && flags[row_l]); m; m &= m - 1) {
+        const uint32_t row = row0 + __ffs(static_cast<int>(m)) - 1;
+        const W* words = buf + static_cast<unsigned long long>(row) * kCosetStride;
+        uint32_t mine = 0;
+        for (uint32_t x = lane; x < kCosetStride; x += 32u) mine += popcount(words[x]);
+        uint32_t upto = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t up = __shfl_up_sync(kFullMask, upto, o);
+          if (lane >= static_cast<uint32_t>(o)) upto += up;
+        }
+        unsigned long long at = 0;
+        if (lane == 31) at = atomicAdd(&p.ctl->collected, static_cast<unsigned long long>(upto));
+        at = __shfl_sync(kFullMask, at, 31) + upto - mine;
+        const RowDecode dec = decode_row(in.m, row, p.start);
+        for (uint32_t x = lane; x < kCosetStride && mine; x += 32u)
+          for (W b = words[x]; b; b &= b - 1, ++at) {
+            const unsigned long long s = decode_state<kWide>(dec, x, lowest_bit(b), p.start, keep);
+            if (at < p.front_cap) p.front[at] = s;
+            if (at < kCosetSmall) r->deepest[at] = s;
+          }
+      }
+    }
+  }
+  if (blockIdx.x) return;
+  const uint32_t kept = exhausted ? min(p.small_count[d], kCosetSmall) : 0u;
+  for (uint32_t k = threadIdx.x; k < kept; k += blockDim.x) {
+    const unsigned long long at = p.small[(d & 1u) * kCosetSmall + k], w = at / 64;
+    const RowDecode dec = decode_row(in.m, static_cast<uint32_t>(w / kCosetStride), p.start);
+    r->previous[k] = decode_state<kWide>(dec, static_cast<uint32_t>(w % kCosetStride), static_cast<uint32_t>(at % 64),
+                                         p.start, keep);
+  }
+  for (uint32_t k = threadIdx.x; k < kReportLayers && k <= d + 1; k += blockDim.x) {
+    r->counts[k] = __ldcg(p.counts + k);
+    r->stamps[k] = p.stamps[k];
+  }
+  if (threadIdx.x == 0) {
+    r->previous_count = kept;
+    r->steps = d + 1;
+    r->error = p.ctl->error;
+  }
+}
+
+// A whole search per launch: step d pulls layer d + 1 of every job, one grid
+// barrier ends it.  A work item is up to `units` units of one job; its warp
+// first looks, one lane per (unit, generator), which parent rows hold anything,
+// and skips units with none (early and last layers touch few rows).
+template <typename W>
+__global__ void __launch_bounds__(kCosetBlock, sizeof(W) == 8 ? 4 : 5) coset_wave_kernel(CosetParams p) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t warps = gridDim.x * kCosetWarps, warp = blockIdx.x * kCosetWarps + (threadIdx.x >> 5);
+  const uint32_t items = p.item_prefix[p.count];
+  const uint32_t unit_mask = p.units - 1u;
+  uint32_t epoch = 0;
+  coset_setup<W>(p);
+  if (!coset_barrier(p, &epoch)) return;
+  coset_table(p);
+  if (!coset_barrier(p, &epoch)) return;
+  CosetInst in = p.inst[0];
+  for (uint32_t d = 0;; ++d) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.stamps[d] = global_ns();
+    const W* cur = static_cast<const W*>(p.buf[d & 1u]);
+    W* nxt = static_cast<W*>(p.buf[(d & 1u) ^ 1u]);
+    const unsigned long long* cur_flags = p.flags[d & 1u];
+    unsigned long long* nxt_flags = p.flags[(d & 1u) ^ 1u];
+    const bool keep = p.report && d && __ldcg(p.counts + d - 1) < kCosetSmall;
+    // The job of the current item; a wave of one job has nothing to look up.
+    uint32_t i = 0, i_end = p.count == 1 ? items : 0u;
+    bool live = p.count == 1;
+    uint32_t found = 0;  // this lane's new states of job i
+    auto flush = [&]() {
+      const uint32_t sum = __reduce_add_sync(kFullMask, found);
+      if (sum && lane == 0) {
+        atomicAdd(p.counts + static_cast<unsigned long long>(i) * p.stride + d + 1, static_cast<unsigned long long>(sum));
+        p.active[d + 1] = 1;
+      }
+      found = 0;
+    };
+    for (uint32_t item = warp; item < items; item += warps) {
+      if (item >= i_end) {
+        if (live) flush();
+        uint32_t lo = 0, hi = p.count;
+        while (hi - lo > 1) {
+          const uint32_t mid = (lo + hi) / 2;
+          if (__ldg(p.item_prefix + mid) <= item) lo = mid;
+          else hi = mid;
+        }
+        i = lo;
+        i_end = p.item_prefix[i + 1];
+        in = p.inst[i];
+        live = __ldcg(p.counts + static_cast<unsigned long long>(i) * p.stride + d) != 0;
+      }
+      if (!live) continue;
+      const uint32_t unit0 = (item - p.item_prefix[i]) * p.units, all_units = in.rows * kCosetParts;
+      // Parents that hold anything, of this lane's unit.
+      const uint32_t my_unit = unit0 + (lane & unit_mask);
+      uint32_t parents = 0, own_cur = 0, own_nxt = 0;
+      if (my_unit < all_units) {
+        const uint32_t row = my_unit / kCosetParts, shift = 8 * (my_unit - row * kCosetParts);
+        const unsigned long long* desc = p.desc + in.desc_off + static_cast<unsigned long long>(row) * in.gens;
+        for (uint32_t g = lane / p.units; g < in.gens; g += 32u / p.units)
+          if (cur_flags[in.row_off + static_cast<uint32_t>(desc[g])]) parents |= 1u << g;
+        own_cur = static_cast<uint32_t>(cur_flags[in.row_off + row] >> shift) & 255u;
+        own_nxt = static_cast<uint32_t>(nxt_flags[in.row_off + row] >> shift) & 255u;
+      }
+      for (uint32_t o = p.units; o < 32u; o <<= 1) parents |= __shfl_xor_sync(kFullMask, parents, o);
+      for (uint32_t u = 0; u < p.units; ++u) {
+        const uint32_t mask = __shfl_sync(kFullMask, parents, u);
+        const uint32_t in_cur = __shfl_sync(kFullMask, own_cur, u), in_nxt = __shfl_sync(kFullMask, own_nxt, u);
+        if (!mask && !in_nxt) continue;  // nothing comes in and nothing is to be cleared
+        const uint32_t unit = unit0 + u, row = unit / kCosetParts, part = unit - row * kCosetParts;
+        const uint32_t x0 = part * 128u + lane;
+        const unsigned long long* desc = p.desc + in.desc_off + static_cast<unsigned long long>(row) * in.gens;
+        W acc[4] = {0, 0, 0, 0};
+        for (uint32_t left = mask; left; left &= left - 1u) {
+          const unsigned long long e = desc[__ffs(static_cast<int>(left)) - 1];
+          const W* from = cur + (in.row_off + static_cast<uint32_t>(e)) * kCosetStride;
+          const uint32_t tau = static_cast<uint32_t>(e >> 32) & 0x1fffu, q = static_cast<uint32_t>(e >> 48);
+          W w[4];
+          if (tau) {
+            const uint16_t* t = p.table + tau * kCosetStride + x0;
+            uint32_t to[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) to[k] = t[32 * k];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[k] = from[to[k] & 1023u];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[k] = flip_inner(w[k], to[k] >> 13);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[k] = from[x0 + 32 * k];
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) acc[k] |= flip_outer(w[k], q);
+        }
+        const unsigned long long own = (in.row_off + row) * kCosetStride + x0;
+        W old[4] = {0, 0, 0, 0};
+        if (in_nxt && (in.inverse_closed || keep)) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) old[k] = nxt[own + 32 * k];
+        }
+        if (in.inverse_closed) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) acc[k] &= ~old[k];
+          if (in_cur && in.same_layer) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[k] &= ~cur[own + 32 * k];
+          }
+        } else if (mask) {
+          W* visited = static_cast<W*>(p.visited) + own;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const W v = visited[32 * k];
+            acc[k] &= ~v;
+            if (acc[k]) visited[32 * k] = v | acc[k];
+          }
+        }
+        if (keep && in_nxt) {
+          // The small layer d - 1 is about to be overwritten.
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            for (W b = old[k]; b; b &= b - 1) {
+              const uint32_t at = atomicAdd(p.small_count + d, 1u);
+              if (at < kCosetSmall) p.small[(d & 1u) * kCosetSmall + at] = (own + 32 * k) * 64ull + lowest_bit(b);
+            }
+        }
+        const bool any = __any_sync(kFullMask, (acc[0] | acc[1] | acc[2] | acc[3]) != 0);
+        if (any || in_nxt) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            nxt[own + 32 * k] = acc[k];
+            found += popcount(acc[k]);
+          }
+          if (lane == 0 && any != (in_nxt != 0))
+            reinterpret_cast<uint8_t*>(nxt_flags + in.row_off + row)[part] = any ? 1 : 0;
+        }
+      }
+    }
+    if (live) flush();
+    if (!coset_barrier(p, &epoch)) return;
+    const bool more = __ldcg(p.active + d + 1) != 0;
+    if (more && d < p.max_steps) continue;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      p.stamps[d + 1] = global_ns();
+      p.ctl->steps = d + 1;
+    }
+    if (blockIdx.x == 0) __syncthreads();
+    if (p.report) coset_finish<W>(p, in, d, !more);
+    return;
+  }
+}
+
+// The deepest layer again, into a buffer that holds it.
+template <typename W>
+__global__ void __launch_bounds__(kCosetBlock) coset_collect(CosetParams p, uint32_t last) {
+  coset_finish<W>(p, p.inst[0], last, true);
+}
+
+size_t al256(size_t x) { return (x + 255) / 256 * 256; }
+
+uint32_t embedded(uint32_t n) { return std::max(n, kSlots); }
+
+size_t table_bytes() { return static_cast<size_t>(kSlotPerms) * kCosetStride * sizeof(uint16_t); }
+
+}  // namespace
+
+bool coset_supported(uint32_t n, uint32_t gens) {
+  return n >= 2 && n <= kCosetMaxDegree && gens >= 1 && gens <= kCosetMaxGens;
+}
+
+uint64_t coset_job_bytes(const CosetJob& job, uint32_t max_depth) {
+  const uint32_t rows = rows_of(embedded(job.n));
+  const uint64_t word = coset_wide(job.n) ? 8 : 4, buffers = job.inverse_closed ? 2 : 3;
+  return rows * (buffers * kCosetStride * word + 16 + 8ull * job.gens) + sizeof(CosetInst) + 4 + 16ull * job.gens +
+         8ull * (max_depth + 2);
+}
+
+uint64_t coset_fixed_bytes(uint32_t max_depth) {
+  return table_bytes() + kSlotPerms + 16ull * kCosetSmall + 16ull * (max_depth + 2) + 32 * 256;
+}
+
+int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_count, cudaStream_t stream,
+               CosetMemory* memory, CosetResult* out, DeviceBuffer* collect, uint64_t start_word) {
+  const uint32_t count = static_cast<uint32_t>(jobs.size());
+  if (!count || !max_depth || (collect && count != 1)) return MGBFS2_INVALID_ARGUMENT;
+  const bool wide = coset_wide(jobs[0].n);
+  const size_t word = wide ? 8 : 4;
+  const void* kernel = wide ? reinterpret_cast<const void*>(coset_wave_kernel<unsigned long long>)
+                            : reinterpret_cast<const void*>(coset_wave_kernel<uint32_t>);
+  int per_sm = 0;
+  MG_CHECK_COSET(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kCosetBlock, 0));
+  if (per_sm < 1) return MGBFS2_UNSUPPORTED;
+  // Units per item: eight, fewer while that leaves warps without an item.
+  uint64_t units = 0;
+  for (const CosetJob& j : jobs) {
+    if (!coset_supported(j.n, j.gens) || coset_wide(j.n) != wide || !j.perms) return MGBFS2_INVALID_ARGUMENT;
+    units += static_cast<uint64_t>(rows_of(embedded(j.n))) * kCosetParts;
+  }
+  const uint64_t warps = static_cast<uint64_t>(per_sm) * sm_count * kCosetWarps;
+  uint32_t per_item = kMaxUnits;
+  while (per_item > 1 && units / per_item < 6 * warps) per_item /= 2;
+  std::vector<CosetInst> inst(count);
+  std::vector<uint32_t> prefix(count + 1, 0);
+  std::vector<uint8_t> perms;
+  unsigned long long rows = 0, descs = 0, visited_rows = 0;
+  for (uint32_t i = 0; i < count; ++i) {
+    const CosetJob& j = jobs[i];
+    CosetInst& c = inst[i];
+    c.m = embedded(j.n);
+    c.gens = j.gens;
+    c.rows = rows_of(c.m);
+    c.inverse_closed = j.inverse_closed;
+    c.same_layer = 0;
+    c.perm_off = static_cast<uint32_t>(perms.size());
+    c.row_off = rows;
+    c.desc_off = descs;
+    for (uint32_t g = 0; g < j.gens; ++g) {
+      const uint32_t* s = j.perms + static_cast<size_t>(g) * j.n;
+      for (uint32_t k = 0; k < 16; ++k) perms.push_back(static_cast<uint8_t>(k < j.n ? s[k] : k));
+      uint32_t swaps = 0, seen = 0;
+      for (uint32_t k = 0; k < j.n; ++k)
+        for (uint32_t at = k; !((seen >> at) & 1u); at = s[at]) {
+          seen |= 1u << at;
+          if (s[at] != k) ++swaps;
+        }
+      if (!(swaps & 1u)) c.same_layer = 1;
+    }
+    rows += c.rows;
+    descs += static_cast<unsigned long long>(c.rows) * c.gens;
+    if (!j.inverse_closed) visited_rows = rows;
+    prefix[i + 1] = prefix[i] + (c.rows * kCosetParts + per_item - 1) / per_item;
+  }
+  // Arena: uploaded block | cleared block (tables of the loop, flags, buffers) | tables.
+  const uint32_t stride = max_depth + 2;
+  size_t off = 0;
+  const auto take = [&off](size_t bytes) {
+    const size_t at = off;
+    off = al256(off + bytes);
+    return at;
+  };
+  const size_t o_inst = take(count * sizeof(CosetInst)), o_prefix = take((count + 1) * 4), o_perms = take(perms.size());
+  const size_t upload = off;
+  const size_t o_counts = take(8ull * count * stride), o_active = take(4ull * stride), o_small_count = take(4ull * stride);
+  const size_t o_ctl = take(sizeof(CosetCtl)), o_used = take(kSlotPerms);
+  const size_t o_flags0 = take(8 * rows), o_flags1 = take(8 * rows);
+  const size_t word_bytes[3] = {rows * kCosetStride * word, rows * kCosetStride * word,
+                                visited_rows * kCosetStride * word};
+  const bool own = word_bytes[0] >= kCosetOwnWords;
+  size_t o_words[3];
+  for (int k = 0; k < 3; ++k) o_words[k] = take(own ? 0 : word_bytes[k]);
+  const size_t cleared = off;
+  const size_t o_stamps = take(8ull * stride), o_small = take(16ull * kCosetSmall), o_table = take(table_bytes());
+  const size_t o_desc = take(8 * descs);
+  int rc = memory->arena.ensure(off, true);
+  for (int k = 0; k < 3 && !rc && own; ++k)
+    if (word_bytes[k]) rc = memory->words[k].ensure(word_bytes[k], true);
+  // Room for a small deepest layer; a larger one is written by a second pass.
+  if (!rc && collect) rc = collect->ensure((kCosetSmall + 2) * 8);
+  if (!rc && collect && !memory->report) rc = pinned_take(sizeof(CosetReport), &memory->report);
+  if (rc) return rc;
+  char* base = static_cast<char*>(memory->arena.ptr);
+  void* words[3];
+  for (int k = 0; k < 3; ++k) words[k] = own ? memory->words[k].ptr : base + o_words[k];
+  std::vector<char> host(upload);
+  std::memcpy(host.data() + o_inst, inst.data(), count * sizeof(CosetInst));
+  std::memcpy(host.data() + o_prefix, prefix.data(), (count + 1) * 4);
+  std::memcpy(host.data() + o_perms, perms.data(), perms.size());
+  CosetParams p{};
+  p.inst = reinterpret_cast<const CosetInst*>(base + o_inst);
+  p.item_prefix = reinterpret_cast<const uint32_t*>(base + o_prefix);
+  p.perms = reinterpret_cast<const uint8_t*>(base + o_perms);
+  p.count = count;
+  p.units = per_item;
+  p.stride = stride;
+  p.max_steps = max_depth - 1;
+  p.counts = reinterpret_cast<unsigned long long*>(base + o_counts);
+  p.active = reinterpret_cast<uint32_t*>(base + o_active);
+  p.stamps = reinterpret_cast<unsigned long long*>(base + o_stamps);
+  p.used = reinterpret_cast<uint8_t*>(base + o_used);
+  p.table = reinterpret_cast<uint16_t*>(base + o_table);
+  p.desc = reinterpret_cast<unsigned long long*>(base + o_desc);
+  p.flags[0] = reinterpret_cast<unsigned long long*>(base + o_flags0);
+  p.flags[1] = reinterpret_cast<unsigned long long*>(base + o_flags1);
+  p.buf[0] = words[0];
+  p.buf[1] = words[1];
+  p.visited = words[2];
+  p.small_count = reinterpret_cast<uint32_t*>(base + o_small_count);
+  p.small = reinterpret_cast<unsigned long long*>(base + o_small);
+  if (collect) {
+    p.report = static_cast<CosetReport*>(memory->report);
+    p.report->steps = 0;
+    p.front = static_cast<unsigned long long*>(collect->ptr);
+    p.front_cap = collect->bytes / 8;
+    p.start = start_word;
+    p.n = jobs[0].n;
+  }
+  p.descs = descs;
+  p.ctl = reinterpret_cast<CosetCtl*>(base + o_ctl);
+  cudaError_t e = cudaMemcpyAsync(base, host.data(), upload, cudaMemcpyHostToDevice, stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(base + upload, 0, cleared - upload, stream);
+  for (int k = 0; k < 3 && own && e == cudaSuccess; ++k)
+    if (word_bytes[k]) e = cudaMemsetAsync(words[k], 0, word_bytes[k], stream);
+  const uint64_t blocks = std::min<uint64_t>((prefix[count] + kCosetWarps - 1) / kCosetWarps,
+                                             static_cast<uint64_t>(per_sm) * sm_count);
+  if (e == cudaSuccess) {
+    void* args[] = {&p};
+    e = cudaLaunchCooperativeKernel(kernel, dim3(static_cast<uint32_t>(blocks)), dim3(kCosetBlock), args, 0, stream);
+  }
+  CosetCtl ctl{};
+  if (e == cudaSuccess && !collect) e = cudaMemcpyAsync(&ctl, p.ctl, sizeof(ctl), cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  if (e != cudaSuccess) return cuda_status(e);
+  if (p.report) {
+    ctl.steps = p.report->steps;
+    ctl.error = ctl.steps ? p.report->error : static_cast<uint32_t>(ERR_WAIT_LIMIT);  // no report: a barrier gave up
+  }
+  out->launches = 1;
+  out->steps = ctl.steps;
+  out->fatal = ctl.error;
+  // Columns 0 .. steps of the layer table, and the step times.
+  const uint32_t cols = std::min(ctl.steps + 1, stride);
+  std::vector<unsigned long long> stamps(cols), counts(static_cast<size_t>(count) * cols);
+  if (p.report && cols <= kReportLayers) {
+    std::memcpy(counts.data(), p.report->counts, 8ull * cols);
+    std::memcpy(stamps.data(), p.report->stamps, 8ull * cols);
+  } else {
+    MG_CHECK_COSET(cudaMemcpy2DAsync(counts.data(), 8ull * cols, p.counts, 8ull * stride, 8ull * cols, count,
+                                     cudaMemcpyDeviceToHost, stream));
+    MG_CHECK_COSET(cudaMemcpyAsync(stamps.data(), p.stamps, 8ull * cols, cudaMemcpyDeviceToHost, stream));
+    MG_CHECK_COSET(cudaStreamSynchronize(stream));
+  }
+  out->layers.assign(count, {});
+  out->overflow.assign(count, 0);
+  for (uint32_t i = 0; i < count; ++i) {
+    const unsigned long long* row = counts.data() + static_cast<size_t>(i) * cols;
+    for (uint32_t d = 0; d < cols && row[d]; ++d) out->layers[i].push_back(row[d]);
+    out->overflow[i] = out->layers[i].size() > max_depth;
+  }
+  out->step_seconds.clear();
+  for (uint32_t d = 0; d + 1 < cols; ++d) out->step_seconds.push_back(static_cast<double>(stamps[d + 1] - stamps[d]) * 1e-9);
+  out->kernel_seconds = cols > 1 ? static_cast<double>(stamps[cols - 1] - stamps[0]) * 1e-9 : 0.0;
+  if (!collect || out->fatal || out->overflow[0]) return MGBFS2_OK;
+  const CosetReport& r = *p.report;
+  out->previous_small.assign(r.previous, r.previous + r.previous_count);
+  const uint64_t deepest = out->layers[0].back();
+  if (deepest <= kCosetSmall) out->deepest_small.assign(r.deepest, r.deepest + deepest);
+  if (deepest <= p.front_cap) return MGBFS2_OK;
+  if ((rc = collect->ensure((deepest + 2) * 8))) return rc;
+  p.front = static_cast<unsigned long long*>(collect->ptr);
+  p.front_cap = deepest;
+  const uint32_t last = ctl.steps - 1;
+  MG_CHECK_COSET(cudaMemsetAsync(&p.ctl->collected, 0, sizeof(unsigned long long), stream));
+  if (wide) coset_collect<unsigned long long><<<static_cast<uint32_t>(blocks), kCosetBlock, 0, stream>>>(p, last);
+  else coset_collect<uint32_t><<<static_cast<uint32_t>(blocks), kCosetBlock, 0, stream>>>(p, last);
+  ++out->launches;
+  MG_CHECK_COSET(cudaGetLastError());
+  MG_CHECK_COSET(cudaStreamSynchronize(stream));
+  return MGBFS2_OK;
+}
+
+}  // namespace mgbfs2

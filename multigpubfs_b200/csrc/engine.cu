@@ -23,6 +23,7 @@
 
 #include "../../include/mgbfs2.h"
 #include "bucket_kernels.cuh"
+#include "coset.h"
 #include "engine.h"
 #include "grouped_kernels.cuh"
 #include "packed_kernels.cuh"
@@ -42,6 +43,7 @@ namespace {
 using Clock = std::chrono::steady_clock;
 
 constexpr uint64_t kRouteChunkAlign = 1024;  // parents: route chunks start 8 KB apart
+constexpr uint32_t kCosetDepth = 4096;       // layers a search in coset-word layers may have
 
 void set_message(char* error, size_t capacity, const std::string& text) {
   if (!error || !capacity) return;
@@ -535,6 +537,11 @@ void Graph::release() {
   for (DeviceBuffer* b : {&bitmap, &front, &next, &table, &bank[0], &bank[1], &bank[2], &program, &control_buf,
                           &scratch, &buckets, &shard_meta, &group_meta, &loop_buf, &transp_buf})
     b->release_to_cache(device);
+  if (coset) {
+    coset->release_to_cache(device);
+    delete coset;
+    coset = nullptr;
+  }
   wide_release();
   if (host_control) {
     pinned_give(host_control);
@@ -1300,9 +1307,19 @@ int Graph::make_plan(const mgbfs2_plan_request* req, mgbfs2_plan_info* out) {
     int rc = wide_plan(&p, budget);
     if (rc) return rc;
   }
+  // The default plan of a Lehmer bitmap runs a whole search in coset-word
+  // layers (coset.h) where their buffers fit: nothing asked for that only the
+  // list layers have (a dedup, a frontier capacity, shapes, the host loop), and
+  // no caller's bound below the rank domain that a layer might have to break.
+  const CosetJob job{elements, gens, perms.data(), inverse_closed};
+  coset_ok = visited == MGBFS2_VISITED_BITMAP && r.dedup == MGBFS2_DEDUP_AUTO && lehmer && !use_product &&
+             !host_loop_only && !r.capacity && !r.shards && !r.group_chunk && !r.blocks_per_sm &&
+             !r.parents_per_thread && !r.route_chunk && !r.bucket_min_work && !r.bucket_margin &&
+             (!orbit_bound || orbit_bound >= rank_total) && coset_supported(elements, gens) &&
+             coset_job_bytes(job, kCosetDepth) + coset_fixed_bytes(kCosetDepth) <= budget / 2;
   // Fixed allocations of the plan.
   int rc = MGBFS2_OK;
-  if (p.visited == MGBFS2_VISITED_BITMAP) rc = bitmap.ensure(bitmap_bytes);
+  if (p.visited == MGBFS2_VISITED_BITMAP && !coset_ok) rc = bitmap.ensure(bitmap_bytes);
   if (!rc) rc = control_buf.ensure(sizeof(Control));
   if (!rc && packed) rc = program.ensure(terms.size() * sizeof(Term) + term_begin.size() * sizeof(uint32_t) + 16);
   if (!rc && !host_control) rc = pinned_take(sizeof(Control), reinterpret_cast<void**>(&host_control));
@@ -2167,11 +2184,83 @@ int Graph::run_device_loop(const void* fn, ExpandParams* pp, size_t smem, uint64
   return MGBFS2_OK;
 }
 
+// A whole search in coset-word layers, from the identity: the layer sizes do
+// not depend on the start, and its states are those of the identity's search
+// with the codes mapped through the start.
+int Graph::coset_run(mgbfs2_status* status) {
+  mgbfs2_status st{};
+  const auto started = Clock::now();
+  MG_CHECK(cudaEventRecord(ev_run[0], stream));
+  CosetResult r;
+  if (!coset) {
+    coset = new CosetMemory();
+    coset->set_stream(stream);
+  }
+  {
+    TraceRange range("layers.coset");
+    const int rc = coset_wave({CosetJob{elements, gens, perms.data(), inverse_closed}}, kCosetDepth, sm_count, stream,
+                              coset, &r, &front, start_word);
+    if (rc) return rc;
+  }
+  if (r.overflow[0]) {  // deeper than its layer table: the list layers have no such limit
+    return run_lists(nullptr, nullptr, nullptr, status);
+  }
+  coset_ran = true;
+  front_grouped = false;
+  layer_sizes = r.layers[0];
+  const uint32_t deepest = static_cast<uint32_t>(layer_sizes.size() - 1);
+  layer_seconds.assign(r.step_seconds.begin(), r.step_seconds.begin() + std::min<size_t>(deepest, r.step_seconds.size()));
+  for (int i = 0; i < 2; ++i) {
+    small_layer[i].clear();
+    small_depth[i] = UINT32_MAX;
+  }
+  if (!r.fatal) {
+    if (deepest && layer_sizes[deepest - 1] < kCosetSmall) keep_small(deepest - 1, std::move(r.previous_small));
+    if (layer_sizes[deepest] < kCosetSmall) keep_small(deepest, std::move(r.deepest_small));
+  }
+  last_count = r.fatal ? 0 : layer_sizes[deepest];
+  launches = r.launches;
+  st.complete = r.fatal == 0;
+  st.reason = r.fatal ? MGBFS2_REASON_RESOURCE : MGBFS2_REASON_FRONTIER_EXHAUSTED;
+  st.fatal = r.fatal;
+  st.layers = deepest + 1;
+  for (uint32_t d = 0; d <= deepest; ++d) {
+    const uint64_t c = layer_sizes[d];
+    st.states += c;
+    st.successors += c * gens;
+    st.visited_tests += c * gens - (parent_skip && d > 0 ? c : 0);
+  }
+  if (cudaEventRecord(ev_run[1], stream) == cudaSuccess && cudaEventSynchronize(ev_run[1]) == cudaSuccess) {
+    float ms = 0.f;
+    if (cudaEventElapsedTime(&ms, ev_run[0], ev_run[1]) == cudaSuccess) st.device_seconds = ms * 1e-3;
+  }
+  st.kernel_seconds = r.kernel_seconds;
+  st.bfs_seconds = std::chrono::duration<double>(Clock::now() - started).count();
+  st.kernel_launches = launches;
+  st.peak_device_bytes = std::max<uint64_t>(plan.device_bytes, coset->bytes() + front.bytes);
+  if (status) *status = st;
+  return MGBFS2_OK;
+}
+
 int Graph::run(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, void* user, mgbfs2_status* status) {
   if (!planned) return MGBFS2_STATE;
   TraceRange range("mgbfs2.run");
   MG_CHECK(cudaSetDevice(device));
   if (!packed) return wide_run(limits, cb, user, status);
+  const bool limited = limits && (limits->max_seconds > 0 || limits->max_layers || limits->cancel);
+  if (coset_ok && !limited && !cb && !resume_pending) return coset_run(status);
+  return run_lists(limits, cb, user, status);
+}
+
+// The layer loop over frontier lists: the device loop or one layer at a time.
+int Graph::run_lists(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, void* user, mgbfs2_status* status) {
+  coset_ran = false;
+  if (coset_ok) {
+    // The plan left the bitmap to the run that needs it, in the place of the
+    // coset-word buffers.
+    if (coset) coset->free();
+    if (int rc = bitmap.ensure((rank_domain() + 63) / 64 * 8)) return rc;
+  }
   mgbfs2_status st{};
   // A resumed run starts from the checkpoint's layer table, deepest layer
   // (in `front`), visited structure and small-layer samples.
@@ -2616,7 +2705,9 @@ int Graph::sample(uint32_t which, int64_t* out, size_t cap_rows, size_t* rows) {
   if (which == 0) {
     const uint64_t n = std::min<uint64_t>(last_count, cap_rows);
     words.resize(n);
-    if (n) {
+    if (n && small_depth[0] == deepest && small_layer[0].size() >= n) {
+      std::copy_n(small_layer[0].begin(), n, words.begin());  // a small layer is on the host already
+    } else if (n) {
       MG_CHECK(cudaMemcpyAsync(words.data(), front.ptr, n * 8, cudaMemcpyDeviceToHost, stream));
       MG_CHECK(cudaStreamSynchronize(stream));
     }

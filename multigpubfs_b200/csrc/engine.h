@@ -66,6 +66,7 @@ uint64_t pool_idle_bytes(int device);
 int device_free_bytes(int device, size_t* free_bytes, bool fresh = false);
 
 struct WideState;     // int64-key arena path (wide.cu)
+struct CosetMemory;   // coset.h
 struct ExpandParams;  // packed_kernels.cuh
 
 // A named NVTX range for the lifetime of the object: a profiler's timeline
@@ -190,6 +191,14 @@ struct Graph {
   bool host_loop_only = false;  // plan option MGBFS2_OPTION_HOST_LOOP
   int run_device_loop(const void* fn, ExpandParams* p, size_t smem, uint64_t cap, mgbfs2_status* st,
                       double* kernel_seconds, uint64_t* count, uint64_t* visited, uint32_t* depth, bool* paused);
+
+  // Coset-word layers (coset.h): the default plan of a Lehmer bitmap runs a
+  // whole unlimited search in them.  coset_ran: `bitmap` does not hold the last
+  // run's visited states (a checkpoint runs the list layers again first).
+  CosetMemory* coset = nullptr;
+  bool coset_ok = false, coset_ran = false;
+  int coset_run(mgbfs2_status* status);
+  int run_lists(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, void* user, mgbfs2_status* status);
 
   // Checkpoint / resume (checkpoint.cu): read_checkpoint restores the visited
   // structure, the deepest layer (in `front`) and the layer table, and the

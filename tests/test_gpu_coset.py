@@ -1,0 +1,98 @@
+"""Coset-word layers (the default plan of a Lehmer bitmap) against the oracle
+and the list layers: every degree from the embedded ones (below 7) through both
+word widths, directed and inverse-closed sets, sets with and without an even
+generator, the smallest and largest number of generators, small orbits."""
+import random
+
+import pytest
+
+from oracle import graph_oracle as G
+from oracle import packed_oracle as P
+
+pytestmark = pytest.mark.gpu
+
+
+def _search(graph, **plan):
+    from multigpubfs_b200 import GraphDefinition
+    from multigpubfs_b200.engine import NativeGraph
+    with NativeGraph(GraphDefinition.from_dict(graph)) as e:
+        e.plan(**plan)
+        r = e.run()
+        return r, e.sample(0, 1000), e.sample(1, 1000)
+
+
+def _generators(rng, n, count, kind):
+    gens = []
+    for _ in range(count):
+        g = list(range(n))
+        if kind == "odd":  # transpositions: no edge inside a layer
+            i, j = rng.sample(range(n), 2)
+            g[i], g[j] = g[j], g[i]
+        elif kind == "cycle":  # one orbit of a cyclic group
+            g = g[1:] + g[:1]
+        else:
+            rng.shuffle(g)
+        gens.append(g)
+    return gens
+
+
+def _closed(gens):
+    out = [list(g) for g in gens]
+    for g in gens:
+        inv = sorted(range(len(g)), key=lambda i: g[i])
+        if inv not in out:
+            out.append(inv)
+    return out
+
+
+@pytest.mark.parametrize("n", range(2, 12))
+@pytest.mark.parametrize("kind", ["any", "odd", "cycle", "closed"])
+def test_matches_the_oracle(n, kind):
+    rng = random.Random(1000 * n + len(kind))
+    for count in (1, 2, 3, 32) if n <= 9 else (2, 4):
+        gens = _generators(rng, n, count, kind)
+        gens = _closed(gens)[:32] if kind == "closed" else gens
+        start = list(range(n))
+        rng.shuffle(start)
+        sizes, last, _ = P.packed_bfs(gens, start, sample=1 << 20)
+        r, current, _ = _search(G.permutation_graph(gens, start))
+        assert r.complete and r.layer_sizes == sizes, (n, kind, count)
+        assert r.successors == len(gens) * sum(sizes)
+        if sizes[-1] <= 1000:
+            assert current == last, (n, kind, count)
+
+
+@pytest.mark.parametrize("n,count,closed", [(7, 3, True), (8, 33, False), (9, 2, False), (10, 2, True), (12, 2, False),
+                                            (12, 4, True), (13, 2, True), (13, 2, False)])
+def test_matches_the_list_layers(n, count, closed):
+    """Tables, samples and counts of the same search in list layers (33
+    generators take them under the default plan too)."""
+    rng = random.Random(n * 100 + count)
+    gens = _generators(rng, n, count, "any")
+    gens = _closed(gens) if closed else gens
+    graph = G.permutation_graph(gens, rng.sample(range(n), n))
+    lists, last, small = _search(graph, visited="bitmap", dedup="bucket" if n > 12 else "atomic")
+    r, current, previous = _search(graph)
+    assert r.layer_sizes == lists.layer_sizes
+    assert (r.successors, r.visited_tests, r.states) == (lists.successors, lists.visited_tests, lists.states)
+    assert previous == small
+    if r.layer_sizes[-1] <= 1000:
+        assert current == last
+
+
+def test_a_finished_search_is_checkpointed_and_read_back(tmp_path):
+    """The checkpoint of a finished search holds the Lehmer bitmap, which the
+    coset-word layers do not make: it loads, and its search is over."""
+    from multigpubfs_b200 import GraphDefinition
+    from multigpubfs_b200.engine import NativeGraph
+    g = GraphDefinition.from_dict(G.permutation_graph(G.lrx_generators(8), [3, 1, 4, 0, 5, 7, 2, 6]))
+    with NativeGraph(g) as e:
+        e.plan()
+        full = e.run()
+        words = sorted(e.frontier_words().tolist())
+        e.checkpoint(tmp_path / "done.bin")
+    with NativeGraph(g) as e:
+        e.plan()
+        e.resume(tmp_path / "done.bin")
+        assert e.run().layer_sizes == full.layer_sizes
+        assert sorted(e.frontier_words().tolist()) == words
