@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "../../include/mgbfs2.h"
+#include "coset.h"
 #include "engine.h"
 
 #define MG_CHECK_BATCH(expr)                          \
@@ -619,6 +620,7 @@ struct Batch {
     std::vector<uint32_t> begin;   // gens + 1 relative offsets
     std::vector<uint32_t> inverse; // gens entries
     std::vector<uint32_t> sel;     // byte-permute selectors (6 per generator); empty = displacement terms
+    std::vector<uint32_t> perms;   // gens x n images
     bool inverse_closed = false;
     uint64_t orbit = 0;            // n!
     std::vector<uint64_t> layers;
@@ -631,6 +633,7 @@ struct Batch {
   int sm_count = 148;
   std::vector<Instance> inst;
   DeviceBuffer arena;
+  CosetMemory coset;
   mgbfs2_batch_status last{};
 };
 
@@ -656,6 +659,7 @@ static int validate_instance(const mgbfs2_graph_desc& d, Batch::Instance* out, s
   in.gens = d.generators;
   in.orbit = factorial(n);
   in.begin.assign(1, 0);
+  in.perms.assign(d.permutations, d.permutations + static_cast<size_t>(in.gens) * n);
   // A generator of at most 15 points is one 60-bit word (4 bits per image), so
   // finding a generator's inverse among them is a word comparison.
   std::vector<uint64_t> words(in.gens);
@@ -743,6 +747,7 @@ static int batch_create(const mgbfs2_graph_desc* graphs, uint32_t count, int dev
     return fail(rc, "CUDA_SETUP");
   }
   b->arena.stream = b->stream;
+  b->coset.set_stream(b->stream);
   retain_pool_memory(device);
   cudaDeviceGetAttribute(&b->sm_count, cudaDevAttrMultiProcessorCount, device);
   *out = b;
@@ -807,6 +812,7 @@ static int run_wave(Batch* b, const std::vector<uint32_t>& ids, const std::vecto
   const size_t o_buf0 = off; off = al(off + (seg + pool) * 8);
   const size_t o_buf1 = off; off = al(off + (seg + pool) * 8);
   // Exact size: waves are planned against the memory budget, so no headroom.
+  b->coset.free();  // a wave of list layers is sized by the whole budget
   int rc = b->arena.ensure(off, true);
   if (rc) return rc;
   char* base = static_cast<char*>(b->arena.ptr);
@@ -971,6 +977,42 @@ static int run_wave(Batch* b, const std::vector<uint32_t>& ids, const std::vecto
   return MGBFS2_OK;
 }
 
+// Runs one wave in coset-word layers (coset.h): every instance to the end in
+// one launch, whatever its layers' sizes.
+static int run_coset_wave(Batch* b, const std::vector<uint32_t>& ids, uint32_t max_depth, mgbfs2_batch_status* st,
+                          double* kernel_seconds) {
+  TraceRange range("batch.coset_wave");
+  std::vector<CosetJob> jobs;
+  for (uint32_t i : ids) {
+    const auto& in = b->inst[i];
+    jobs.push_back(CosetJob{in.n, in.gens, in.perms.data(), in.inverse_closed});
+  }
+  CosetResult r;
+  b->arena.free();
+  if (int rc = coset_wave(jobs, max_depth, b->sm_count, b->stream, &b->coset, &r)) return rc;
+  st->kernel_launches += r.launches;
+  st->layer_steps += r.steps;
+  *kernel_seconds += r.kernel_seconds;
+  for (size_t k = 0; k < ids.size(); ++k) {
+    auto& in = b->inst[ids[k]];
+    in.runs++;
+    in.layers.clear();
+    in.layer_seconds.clear();
+    if (r.fatal) continue;  // a barrier gave up: the instance stays incomplete
+    if (r.overflow[k]) {
+      in.status = INST_OVERFLOW;
+      st->fatal |= ERR_FRONTIER_OVERFLOW;
+      continue;
+    }
+    in.status = INST_DONE;
+    in.layers = std::move(r.layers[k]);
+    in.layer_seconds.assign(1, 0.0);
+    for (size_t d = 1; d < in.layers.size(); ++d) in.layer_seconds.push_back(r.step_seconds[d - 1]);
+  }
+  st->fatal |= r.fatal;
+  return MGBFS2_OK;
+}
+
 }  // namespace mgbfs2
 
 using mgbfs2::Batch;
@@ -1008,7 +1050,7 @@ int mgbfs2_batch_run(mgbfs2_batch* batch, const mgbfs2_batch_options* options, m
   MG_CHECK_BATCH(cudaSetDevice(b->device));
   size_t free_bytes = 0;
   if (int frc = device_free_bytes(b->device, &free_bytes)) return frc;
-  free_bytes += pool_idle_bytes(b->device) + device_cache_bytes(b->device) + b->arena.bytes;
+  free_bytes += pool_idle_bytes(b->device) + device_cache_bytes(b->device) + b->arena.bytes + b->coset.bytes();
   const uint64_t reserve = o.reserve_bytes ? o.reserve_bytes : (2ull << 30);
   uint64_t budget = o.memory_bytes ? o.memory_bytes : (free_bytes > reserve ? free_bytes - reserve : 0);
   mgbfs2_batch_status st{};
@@ -1060,7 +1102,31 @@ int mgbfs2_batch_run(mgbfs2_batch* batch, const mgbfs2_batch_options* options, m
     // released its bit counts again), so its redo segments rarely sum to more
     // than twice its orbit; a pool that runs out falls back to the rerun.
     const uint64_t pool = predicted && short_by && budget > used ? std::min((budget - used) / 16, 2 * orbits) : 0;
-    rc = run_wave(b, wave, caps, pool, max_depth, blocks_per_sm, tile_ppt, loop, &st, &kernel_seconds);
+    // A default sweep (no shapes, no predicted capacities, the persistent loop)
+    // of instances that coset-word layers take runs in them; of a wave that
+    // mixes word widths (degrees up to 12, 13 and 14) only the first instance's
+    // width, the rest in a later wave.  A degree-15 instance keeps its wave in
+    // list layers.
+    bool coset = loop == kLoopPersistent && !blocks_per_sm && !o.tile_entries && !predicted;
+    for (uint32_t i : wave) coset = coset && coset_supported(b->inst[i].n, b->inst[i].gens);
+    if (coset) {
+      std::vector<uint32_t> same;
+      uint64_t need = coset_fixed_bytes(max_depth);
+      for (uint32_t i : wave) {
+        const auto& in = b->inst[i];
+        if (coset_wide(in.n) != coset_wide(b->inst[wave[0]].n)) {
+          later.push_back(i);
+          continue;
+        }
+        same.push_back(i);
+        need += coset_job_bytes(CosetJob{in.n, in.gens, nullptr, in.inverse_closed}, max_depth);
+      }
+      if (need <= budget) wave.swap(same);
+      else coset = false;
+      if (!coset) later.resize(later.size() - (wave.size() - same.size()));
+    }
+    rc = coset ? run_coset_wave(b, wave, max_depth, &st, &kernel_seconds)
+               : run_wave(b, wave, caps, pool, max_depth, blocks_per_sm, tile_ppt, loop, &st, &kernel_seconds);
     ++st.waves;
     for (uint32_t i : wave) {
       if (b->inst[i].status == INST_OVERFLOW) {
@@ -1136,6 +1202,7 @@ void mgbfs2_batch_destroy(mgbfs2_batch* batch) {
   // device cache, where the next batch or graph handle takes it.
   if (b->stream) cudaStreamSynchronize(b->stream);
   b->arena.release_to_cache(b->device);
+  b->coset.release_to_cache(b->device);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
   delete batch;

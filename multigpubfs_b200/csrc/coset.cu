@@ -49,9 +49,10 @@ struct CosetParams {
   uint32_t stride, max_steps;   // layer-table columns; last step that may run
   unsigned long long* counts;   // count x stride layer sizes
   uint32_t* active;             // stride: layer d of any job is not empty
+  uint32_t* next_item;          // stride: work items of step d taken so far, past the first of every warp
   unsigned long long* stamps;   // stride: globaltimer at the start of step d
   uint8_t* used;                // slot permutations that some row needs
-  uint16_t* table;              // slot permutation x node -> node | flips << 13
+  uint32_t* table;              // slot permutation x node -> image and flips (table_entry)
   unsigned long long* desc;     // row x generator -> parent row | slot permutation << 32 | outer flips << 48
   unsigned long long* flags[2]; // per row: byte p = part p of the buffer's row is not zero
   void* buf[2];
@@ -264,7 +265,7 @@ __device__ __forceinline__ bool coset_barrier(const CosetParams& p, uint32_t* ep
 // the start states.  The parent of a state under g has the label of position p
 // at position g[p].
 template <typename W>
-__device__ void coset_setup(const CosetParams& p) {
+__global__ void __launch_bounds__(kCosetBlock) coset_setup(CosetParams p) {
   const unsigned long long step = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
   const unsigned long long thread = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x;
   for (unsigned long long t = thread; t < p.descs; t += step) {
@@ -308,8 +309,20 @@ __device__ void coset_setup(const CosetParams& p) {
   if (thread == 0) p.active[0] = 1;
 }
 
+// A table entry in the form the pull uses without unpacking: the byte permute
+// selector of the inner flips in the low half (of the low word; the high
+// word's is it ^ 0x4444), the node's image in the high half.  32-bit words keep
+// the lowest flip as a nibble shift of 4 in bits 16..20 and XOR bytes by the
+// other two; 64-bit words XOR bytes by all three.
+template <typename W>
+__device__ __forceinline__ uint32_t table_entry(uint32_t node, uint32_t flips) {
+  if constexpr (sizeof(W) == 8) return (node << 21) | (0x3210u ^ (flips * 0x1111u));
+  else return (node << 21) | ((flips & 1u) << 18) | (0x3210u ^ ((flips >> 1) * 0x1111u));
+}
+
 // The table rows of the slot permutations that some row needs: the image of
 // every node and its inner flips.  One warp takes a permutation.
+template <typename W>
 __device__ void coset_table(const CosetParams& p) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warps = gridDim.x * kCosetWarps, warp = blockIdx.x * kCosetWarps + (threadIdx.x >> 5);
@@ -331,7 +344,7 @@ __device__ void coset_table(const CosetParams& p) {
         seen |= 1u << to;
       }
       for (uint32_t x = lane; x < kCosetStride; x += 32) {
-        uint32_t out = x;  // words past the nodes stay zero and map to themselves
+        uint32_t out = table_entry<W>(x, 0);  // words past the nodes stay zero and map to themselves
         if (x < kCosetNodes) {
           const uint32_t slots = kNodeSlots.at[x];
           uint32_t used = 0, to = 0, flips = 0;
@@ -345,23 +358,24 @@ __device__ void coset_table(const CosetParams& p) {
             to = to * (c * (c - 1) / 2) + j * (j - 1) / 2 + i;
             used |= (1u << a) | (1u << b);
           }
-          out = to | (flips << 13);
+          out = table_entry<W>(to, flips);
         }
-        p.table[perm * kCosetStride + x] = static_cast<uint16_t>(out);
+        p.table[perm * kCosetStride + x] = out;
       }
     }
   }
 }
 
-// Word with its bit index XORed: inner flips r (per lane), outer flips q (uniform).
-__device__ __forceinline__ uint32_t flip_inner(uint32_t w, uint32_t r) {
-  w = __byte_perm(w, 0u, 0x3210u ^ ((r >> 1) * 0x1111u));
-  const uint32_t s = ((w & 0x0f0f0f0fu) << 4) | ((w >> 4) & 0x0f0f0f0fu);
-  return r & 1u ? s : w;
+// Word with its bit index XORed: inner flips of a table entry (per lane),
+// outer flips q (uniform).
+__device__ __forceinline__ uint32_t flip_inner(uint32_t w, uint32_t entry) {
+  w = __byte_perm(w, 0u, entry);
+  const uint32_t by = entry >> 16;  // shifts use the low five bits: 0 or 4
+  return (__funnelshift_l(0u, w, by) & 0xf0f0f0f0u) | (__funnelshift_r(w, 0u, by) & 0x0f0f0f0fu);
 }
-__device__ __forceinline__ unsigned long long flip_inner(unsigned long long w, uint32_t r) {
-  const uint32_t lo = static_cast<uint32_t>(w), hi = static_cast<uint32_t>(w >> 32), x = r * 0x1111u;
-  return (static_cast<unsigned long long>(__byte_perm(lo, hi, 0x7654u ^ x)) << 32) | __byte_perm(lo, hi, 0x3210u ^ x);
+__device__ __forceinline__ unsigned long long flip_inner(unsigned long long w, uint32_t entry) {
+  const uint32_t lo = static_cast<uint32_t>(w), hi = static_cast<uint32_t>(w >> 32);
+  return (static_cast<unsigned long long>(__byte_perm(lo, hi, entry ^ 0x4444u)) << 32) | __byte_perm(lo, hi, entry);
 }
 __device__ __forceinline__ uint32_t swap_bits(uint32_t w, uint32_t mask, int by) {
   return ((w & mask) << by) | ((w >> by) & mask);
@@ -449,15 +463,13 @@ __device__ void coset_finish(const CosetParams& p, const CosetInst& in, uint32_t
 // first looks, one lane per (unit, generator), which parent rows hold anything,
 // and skips units with none (early and last layers touch few rows).
 template <typename W>
-__global__ void __launch_bounds__(kCosetBlock, sizeof(W) == 8 ? 4 : 5) coset_wave_kernel(CosetParams p) {
+__global__ void __launch_bounds__(kCosetBlock, 4) coset_wave_kernel(CosetParams p) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warps = gridDim.x * kCosetWarps, warp = blockIdx.x * kCosetWarps + (threadIdx.x >> 5);
   const uint32_t items = p.item_prefix[p.count];
   const uint32_t unit_mask = p.units - 1u;
   uint32_t epoch = 0;
-  coset_setup<W>(p);
-  if (!coset_barrier(p, &epoch)) return;
-  coset_table(p);
+  coset_table<W>(p);
   if (!coset_barrier(p, &epoch)) return;
   CosetInst in = p.inst[0];
   for (uint32_t d = 0;; ++d) {
@@ -479,7 +491,22 @@ __global__ void __launch_bounds__(kCosetBlock, sizeof(W) == 8 ? 4 : 5) coset_wav
       }
       found = 0;
     };
-    for (uint32_t item = warp; item < items; item += warps) {
+    // Items are taken from a counter, the next one asked for before the current
+    // one is worked on: parents differ too much in what they hold for a fixed
+    // split (S12, six random generators: 30 % of the warps' time went into
+    // waiting at the barrier), and warps that stay close together find each
+    // other's rows in L2 (S13, adjacent transpositions: 54.6 ms, 67.4 ms with
+    // three quarters of the items fixed).  A layer with fewer states than items
+    // skips nearly all of them, which the counter would only slow (S13: 39 ->
+    // 67 us for an empty one): those go round the warps.
+    const bool counter = p.count > 1 || __ldcg(p.counts + d) >= items;
+    uint32_t item = warp;
+    for (uint32_t coming; item < items; item = coming) {
+      coming = item + warps;
+      if (counter) {
+        if (lane == 0) coming = warps + atomicAdd(p.next_item + d, 1u);
+        coming = __shfl_sync(kFullMask, coming, 0);
+      }
       if (item >= i_end) {
         if (live) flush();
         uint32_t lo = 0, hi = p.count;
@@ -502,7 +529,7 @@ __global__ void __launch_bounds__(kCosetBlock, sizeof(W) == 8 ? 4 : 5) coset_wav
         const uint32_t row = my_unit / kCosetParts, shift = 8 * (my_unit - row * kCosetParts);
         const unsigned long long* desc = p.desc + in.desc_off + static_cast<unsigned long long>(row) * in.gens;
         for (uint32_t g = lane / p.units; g < in.gens; g += 32u / p.units)
-          if (cur_flags[in.row_off + static_cast<uint32_t>(desc[g])]) parents |= 1u << g;
+          if (cur_flags[in.row_off + static_cast<uint32_t>(__ldg(desc + g))]) parents |= 1u << g;
         own_cur = static_cast<uint32_t>(cur_flags[in.row_off + row] >> shift) & 255u;
         own_nxt = static_cast<uint32_t>(nxt_flags[in.row_off + row] >> shift) & 255u;
       }
@@ -513,28 +540,49 @@ __global__ void __launch_bounds__(kCosetBlock, sizeof(W) == 8 ? 4 : 5) coset_wav
         if (!mask && !in_nxt) continue;  // nothing comes in and nothing is to be cleared
         const uint32_t unit = unit0 + u, row = unit / kCosetParts, part = unit - row * kCosetParts;
         const uint32_t x0 = part * 128u + lane;
-        const unsigned long long* desc = p.desc + in.desc_off + static_cast<unsigned long long>(row) * in.gens;
+        // Lane g holds generator g's descriptor.
+        uint32_t from_row = 0, how = 0;  // parent row; slot permutation | outer flips << 16
+        if (lane < in.gens) {
+          const unsigned long long e =
+              __ldg(p.desc + in.desc_off + static_cast<unsigned long long>(row) * in.gens + lane);
+          from_row = static_cast<uint32_t>(e);
+          how = static_cast<uint32_t>(e >> 32);
+        }
+        // Generators that keep the free positions' order read the parent row
+        // as it lies; the others through their table row, two at a time, so
+        // that eight gathers are in flight.
+        const uint32_t moved = __ballot_sync(kFullMask, (how & 0xffffu) != 0) & mask, kept = mask & ~moved;
         W acc[4] = {0, 0, 0, 0};
-        for (uint32_t left = mask; left; left &= left - 1u) {
-          const unsigned long long e = desc[__ffs(static_cast<int>(left)) - 1];
-          const W* from = cur + (in.row_off + static_cast<uint32_t>(e)) * kCosetStride;
-          const uint32_t tau = static_cast<uint32_t>(e >> 32) & 0x1fffu, q = static_cast<uint32_t>(e >> 48);
+        for (uint32_t left = kept; left; left &= left - 1u) {
+          const int g = __ffs(static_cast<int>(left)) - 1;
+          const uint32_t q = __shfl_sync(kFullMask, how, g) >> 16;
+          const W* from = cur + (in.row_off + __shfl_sync(kFullMask, from_row, g)) * kCosetStride + x0;
           W w[4];
-          if (tau) {
-            const uint16_t* t = p.table + tau * kCosetStride + x0;
-            uint32_t to[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) to[k] = t[32 * k];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) w[k] = from[to[k] & 1023u];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) w[k] = flip_inner(w[k], to[k] >> 13);
-          } else {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) w[k] = from[x0 + 32 * k];
-          }
+          for (int k = 0; k < 4; ++k) w[k] = from[32 * k];
 #pragma unroll
           for (int k = 0; k < 4; ++k) acc[k] |= flip_outer(w[k], q);
+        }
+        for (uint32_t left = moved; left;) {
+          const int g = __ffs(static_cast<int>(left)) - 1;
+          left &= left - 1u;
+          const int h = left ? __ffs(static_cast<int>(left)) - 1 : g;  // an odd one out is taken twice
+          left &= left - 1u;
+          const uint32_t how_g = __shfl_sync(kFullMask, how, g), how_h = __shfl_sync(kFullMask, how, h);
+          const W* from_g = cur + (in.row_off + __shfl_sync(kFullMask, from_row, g)) * kCosetStride;
+          const W* from_h = cur + (in.row_off + __shfl_sync(kFullMask, from_row, h)) * kCosetStride;
+          const uint32_t* table_g = p.table + (how_g & 0xffffu) * kCosetStride + x0;
+          const uint32_t* table_h = p.table + (how_h & 0xffffu) * kCosetStride + x0;
+          uint32_t to_g[4], to_h[4];
+          W w_g[4], w_h[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) to_g[k] = table_g[32 * k], to_h[k] = table_h[32 * k];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) w_g[k] = from_g[to_g[k] >> 21], w_h[k] = from_h[to_h[k] >> 21];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) acc[k] |= flip_outer(flip_inner(w_g[k], to_g[k]), how_g >> 16);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) acc[k] |= flip_outer(flip_inner(w_h[k], to_h[k]), how_h >> 16);
         }
         const unsigned long long own = (in.row_off + row) * kCosetStride + x0;
         W old[4] = {0, 0, 0, 0};
@@ -603,7 +651,7 @@ size_t al256(size_t x) { return (x + 255) / 256 * 256; }
 
 uint32_t embedded(uint32_t n) { return std::max(n, kSlots); }
 
-size_t table_bytes() { return static_cast<size_t>(kSlotPerms) * kCosetStride * sizeof(uint16_t); }
+size_t table_bytes() { return static_cast<size_t>(kSlotPerms) * kCosetStride * sizeof(uint32_t); }
 
 }  // namespace
 
@@ -619,7 +667,7 @@ uint64_t coset_job_bytes(const CosetJob& job, uint32_t max_depth) {
 }
 
 uint64_t coset_fixed_bytes(uint32_t max_depth) {
-  return table_bytes() + kSlotPerms + 16ull * kCosetSmall + 16ull * (max_depth + 2) + 32 * 256;
+  return table_bytes() + kSlotPerms + 16ull * kCosetSmall + 20ull * (max_depth + 2) + 32 * 256;
 }
 
 int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_count, cudaStream_t stream,
@@ -683,7 +731,7 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   };
   const size_t o_inst = take(count * sizeof(CosetInst)), o_prefix = take((count + 1) * 4), o_perms = take(perms.size());
   const size_t upload = off;
-  const size_t o_counts = take(8ull * count * stride), o_active = take(4ull * stride), o_small_count = take(4ull * stride);
+  const size_t o_counts = take(8ull * count * stride), o_active = take(4ull * stride), o_next = take(4ull * stride), o_small_count = take(4ull * stride);
   const size_t o_ctl = take(sizeof(CosetCtl)), o_used = take(kSlotPerms);
   const size_t o_flags0 = take(8 * rows), o_flags1 = take(8 * rows);
   const size_t word_bytes[3] = {rows * kCosetStride * word, rows * kCosetStride * word,
@@ -718,9 +766,10 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   p.max_steps = max_depth - 1;
   p.counts = reinterpret_cast<unsigned long long*>(base + o_counts);
   p.active = reinterpret_cast<uint32_t*>(base + o_active);
+  p.next_item = reinterpret_cast<uint32_t*>(base + o_next);
   p.stamps = reinterpret_cast<unsigned long long*>(base + o_stamps);
   p.used = reinterpret_cast<uint8_t*>(base + o_used);
-  p.table = reinterpret_cast<uint16_t*>(base + o_table);
+  p.table = reinterpret_cast<uint32_t*>(base + o_table);
   p.desc = reinterpret_cast<unsigned long long*>(base + o_desc);
   p.flags[0] = reinterpret_cast<unsigned long long*>(base + o_flags0);
   p.flags[1] = reinterpret_cast<unsigned long long*>(base + o_flags1);
@@ -746,6 +795,13 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   const uint64_t blocks = std::min<uint64_t>((prefix[count] + kCosetWarps - 1) / kCosetWarps,
                                              static_cast<uint64_t>(per_sm) * sm_count);
   if (e == cudaSuccess) {
+    const uint32_t setup = static_cast<uint32_t>(
+        std::min<unsigned long long>((descs + kCosetBlock - 1) / kCosetBlock, 8ull * static_cast<uint32_t>(sm_count)));
+    if (wide) coset_setup<unsigned long long><<<setup, kCosetBlock, 0, stream>>>(p);
+    else coset_setup<uint32_t><<<setup, kCosetBlock, 0, stream>>>(p);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) {
     void* args[] = {&p};
     e = cudaLaunchCooperativeKernel(kernel, dim3(static_cast<uint32_t>(blocks)), dim3(kCosetBlock), args, 0, stream);
   }
@@ -757,7 +813,7 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
     ctl.steps = p.report->steps;
     ctl.error = ctl.steps ? p.report->error : static_cast<uint32_t>(ERR_WAIT_LIMIT);  // no report: a barrier gave up
   }
-  out->launches = 1;
+  out->launches = 2;
   out->steps = ctl.steps;
   out->fatal = ctl.error;
   // Columns 0 .. steps of the layer table, and the step times.

@@ -96,3 +96,26 @@ def test_a_finished_search_is_checkpointed_and_read_back(tmp_path):
         e.resume(tmp_path / "done.bin")
         assert e.run().layer_sizes == full.layer_sizes
         assert sorted(e.frontier_words().tolist()) == words
+
+
+def test_a_sweep_of_every_degree_and_width():
+    """One batch of degrees 2 to 13, directed and closed: 32- and 64-bit words
+    take separate waves; a degree-13 instance with predicted capacities keeps
+    list layers and gives the same tables."""
+    from multigpubfs_b200.batch import BatchSweep
+    rng = random.Random(5)
+    graphs = []
+    for n in (13, 2, 3, 6, 7, 8, 9, 10, 13, 11):
+        gens = _generators(rng, n, 2, "any")
+        graphs.append(G.permutation_graph(_closed(gens) if n % 2 else gens, rng.sample(range(n), n)))
+    with BatchSweep(graphs) as sweep:
+        st = sweep.run()
+        tables = sweep.layer_tables()
+        assert st["complete_instances"] == len(graphs) and st["waves"] == 2 and st["fatal"] == 0
+        for g, table in zip(graphs, tables):
+            if len(g["start"]) <= 10:
+                assert table == P.packed_bfs(g["action"]["generators"], g["start"])[0]
+        sweep.run(capacities=[1 << 30] * len(graphs))
+        assert sweep.layer_tables() == tables
+        with pytest.raises(Exception):
+            sweep.run(max_depth=4)
