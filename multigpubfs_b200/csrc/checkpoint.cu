@@ -115,8 +115,8 @@ int Graph::write_checkpoint(const char* path) {
   if (!checkpointable(visit)) return MGBFS2_UNSUPPORTED;
   MG_CHECK(cudaSetDevice(device));
   MG_CHECK(cudaStreamSynchronize(stream));
-  if (coset_ran) {
-    // A complete search in coset-word layers left no Lehmer bitmap.
+  if (no_bitmap) {
+    // A complete search without frontier lists left no rank bitmap.
     if (int rc = run_lists(nullptr, nullptr, nullptr, nullptr)) return rc;
   }
   if (front_grouped) {

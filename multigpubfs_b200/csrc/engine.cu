@@ -27,6 +27,7 @@
 #include "engine.h"
 #include "grouped_kernels.cuh"
 #include "packed_kernels.cuh"
+#include "ring.h"
 
 namespace mgbfs2 {
 
@@ -43,7 +44,6 @@ namespace {
 using Clock = std::chrono::steady_clock;
 
 constexpr uint64_t kRouteChunkAlign = 1024;  // parents: route chunks start 8 KB apart
-constexpr uint32_t kCosetDepth = 4096;       // layers a search in coset-word layers may have
 
 void set_message(char* error, size_t capacity, const std::string& text) {
   if (!error || !capacity) return;
@@ -541,6 +541,11 @@ void Graph::release() {
     coset->release_to_cache(device);
     delete coset;
     coset = nullptr;
+  }
+  if (ring) {
+    ring->release_to_cache(device);
+    delete ring;
+    ring = nullptr;
   }
   wide_release();
   if (host_control) {
@@ -1316,7 +1321,17 @@ int Graph::make_plan(const mgbfs2_plan_request* req, mgbfs2_plan_info* out) {
              !host_loop_only && !r.capacity && !r.shards && !r.group_chunk && !r.blocks_per_sm &&
              !r.parents_per_thread && !r.route_chunk && !r.bucket_min_work && !r.bucket_margin &&
              (!orbit_bound || orbit_bound >= rank_total) && coset_supported(elements, gens) &&
-             coset_job_bytes(job, kCosetDepth) + coset_fixed_bytes(kCosetDepth) <= budget / 2;
+             coset_job_bytes(job, kWholeDepth) + coset_fixed_bytes(kWholeDepth) <= budget / 2;
+  // Likewise 2x2 matrices over a prime field in scalar-ring layers (ring.h),
+  // from the layer on where they overtake the list layers.
+  bool ring_field = packed_matrix && rows == 2 && cols == 2 && moduli[0] >= kRingMinPrime &&
+                    moduli[0] <= kRingMaxPrime && start_word;
+  for (uint32_t q = 2; ring_field && q * q <= moduli[0]; ++q) ring_field = moduli[0] % q != 0;
+  ring_ok = ring_field && visited == MGBFS2_VISITED_BITMAP && r.dedup == MGBFS2_DEDUP_AUTO && inverse_closed &&
+            !host_loop_only && !r.capacity && !r.shards && !r.blocks_per_sm && !r.parents_per_thread &&
+            !r.route_chunk && !r.bucket_min_work && !r.bucket_margin && gens <= kRingMaxGens &&
+            (!orbit_bound || orbit_bound >= rank_total) &&
+            ring_bytes(moduli[0], kWholeDepth) + bitmap_bytes <= budget / 2;
   // Fixed allocations of the plan.
   int rc = MGBFS2_OK;
   if (p.visited == MGBFS2_VISITED_BITMAP && !coset_ok) rc = bitmap.ensure(bitmap_bytes);
@@ -2184,77 +2199,23 @@ int Graph::run_device_loop(const void* fn, ExpandParams* pp, size_t smem, uint64
   return MGBFS2_OK;
 }
 
-// A whole search in coset-word layers, from the identity: the layer sizes do
-// not depend on the start, and its states are those of the identity's search
-// with the codes mapped through the start.
-int Graph::coset_run(mgbfs2_status* status) {
-  mgbfs2_status st{};
-  const auto started = Clock::now();
-  MG_CHECK(cudaEventRecord(ev_run[0], stream));
-  CosetResult r;
-  if (!coset) {
-    coset = new CosetMemory();
-    coset->set_stream(stream);
-  }
-  {
-    TraceRange range("layers.coset");
-    const int rc = coset_wave({CosetJob{elements, gens, perms.data(), inverse_closed}}, kCosetDepth, sm_count, stream,
-                              coset, &r, &front, start_word);
-    if (rc) return rc;
-  }
-  if (r.overflow[0]) {  // deeper than its layer table: the list layers have no such limit
-    return run_lists(nullptr, nullptr, nullptr, status);
-  }
-  coset_ran = true;
-  front_grouped = false;
-  layer_sizes = r.layers[0];
-  const uint32_t deepest = static_cast<uint32_t>(layer_sizes.size() - 1);
-  layer_seconds.assign(r.step_seconds.begin(), r.step_seconds.begin() + std::min<size_t>(deepest, r.step_seconds.size()));
-  for (int i = 0; i < 2; ++i) {
-    small_layer[i].clear();
-    small_depth[i] = UINT32_MAX;
-  }
-  if (!r.fatal) {
-    if (deepest && layer_sizes[deepest - 1] < kCosetSmall) keep_small(deepest - 1, std::move(r.previous_small));
-    if (layer_sizes[deepest] < kCosetSmall) keep_small(deepest, std::move(r.deepest_small));
-  }
-  last_count = r.fatal ? 0 : layer_sizes[deepest];
-  launches = r.launches;
-  st.complete = r.fatal == 0;
-  st.reason = r.fatal ? MGBFS2_REASON_RESOURCE : MGBFS2_REASON_FRONTIER_EXHAUSTED;
-  st.fatal = r.fatal;
-  st.layers = deepest + 1;
-  for (uint32_t d = 0; d <= deepest; ++d) {
-    const uint64_t c = layer_sizes[d];
-    st.states += c;
-    st.successors += c * gens;
-    st.visited_tests += c * gens - (parent_skip && d > 0 ? c : 0);
-  }
-  if (cudaEventRecord(ev_run[1], stream) == cudaSuccess && cudaEventSynchronize(ev_run[1]) == cudaSuccess) {
-    float ms = 0.f;
-    if (cudaEventElapsedTime(&ms, ev_run[0], ev_run[1]) == cudaSuccess) st.device_seconds = ms * 1e-3;
-  }
-  st.kernel_seconds = r.kernel_seconds;
-  st.bfs_seconds = std::chrono::duration<double>(Clock::now() - started).count();
-  st.kernel_launches = launches;
-  st.peak_device_bytes = std::max<uint64_t>(plan.device_bytes, coset->bytes() + front.bytes);
-  if (status) *status = st;
-  return MGBFS2_OK;
-}
-
 int Graph::run(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, void* user, mgbfs2_status* status) {
   if (!planned) return MGBFS2_STATE;
   TraceRange range("mgbfs2.run");
   MG_CHECK(cudaSetDevice(device));
   if (!packed) return wide_run(limits, cb, user, status);
   const bool limited = limits && (limits->max_seconds > 0 || limits->max_layers || limits->cancel);
-  if (coset_ok && !limited && !cb && !resume_pending) return coset_run(status);
+  if (!limited && !cb && !resume_pending) {
+    if (coset_ok) return coset_run(status);
+    if (ring_ok) return ring_run(status);
+  }
   return run_lists(limits, cb, user, status);
 }
 
 // The layer loop over frontier lists: the device loop or one layer at a time.
 int Graph::run_lists(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, void* user, mgbfs2_status* status) {
-  coset_ran = false;
+  no_bitmap = false;
+  if (ring) ring->free();
   if (coset_ok) {
     // The plan left the bitmap to the run that needs it, in the place of the
     // coset-word buffers.
@@ -2365,7 +2326,7 @@ int Graph::run_lists(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, 
   // no limits and no callback.
   const bool limited = limits && (limits->max_seconds > 0 || limits->max_layers || limits->cancel);
   const uint64_t loop_cap = std::max<uint64_t>(1, plan.capacity);
-  bool device_loop = !host_loop_only && !bucketed && !grouped_mode && !limited && !cb &&
+  bool device_loop = !host_loop_only && !list_stop && !bucketed && !grouped_mode && !limited && !cb &&
                      (bitmap_kind(visit) || visit == V_HASH || visit == V_HASHQ) &&
                      2 * (loop_cap + 2) * 8 <= (16ull << 30);
   // The device loop never grows the table: it must hold every state below
@@ -2444,7 +2405,8 @@ int Graph::run_lists(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, 
     const double elapsed = std::chrono::duration<double>(Clock::now() - started).count();
     if (limits && limits->cancel && *limits->cancel) { st.reason = MGBFS2_REASON_CANCELLED; break; }
     if (limits && limits->max_seconds > 0 && elapsed >= limits->max_seconds) { st.reason = MGBFS2_REASON_DEADLINE; break; }
-    if (limits && limits->max_layers && layer_sizes.size() >= limits->max_layers) {
+    if ((limits && limits->max_layers && layer_sizes.size() >= limits->max_layers) ||
+        (list_stop && count >= list_stop)) {
       st.reason = MGBFS2_REASON_LAYER_LIMIT;
       break;
     }

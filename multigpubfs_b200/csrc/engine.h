@@ -15,6 +15,8 @@ namespace mgbfs2 {
 
 int cuda_status(cudaError_t e);
 
+constexpr uint32_t kWholeDepth = 4096;  // layers a search without frontier lists may have
+
 // Sets fn's shared-memory carveout on the current device to the smallest
 // configuration that holds `want` resident blocks of `threads` threads (fewer
 // where registers or shared memory allow fewer), leaving the rest as L1.
@@ -67,6 +69,7 @@ int device_free_bytes(int device, size_t* free_bytes, bool fresh = false);
 
 struct WideState;     // int64-key arena path (wide.cu)
 struct CosetMemory;   // coset.h
+struct RingMemory;    // ring.h
 struct ExpandParams;  // packed_kernels.cuh
 
 // A named NVTX range for the lifetime of the object: a profiler's timeline
@@ -192,12 +195,16 @@ struct Graph {
   int run_device_loop(const void* fn, ExpandParams* p, size_t smem, uint64_t cap, mgbfs2_status* st,
                       double* kernel_seconds, uint64_t* count, uint64_t* visited, uint32_t* depth, bool* paused);
 
-  // Coset-word layers (coset.h): the default plan of a Lehmer bitmap runs a
-  // whole unlimited search in them.  coset_ran: `bitmap` does not hold the last
-  // run's visited states (a checkpoint runs the list layers again first).
+  // Searches without frontier lists (whole_search.cu): the default plan of a
+  // Lehmer bitmap in coset-word layers (coset.h), of 2x2 matrices over a prime
+  // field in scalar-ring layers (ring.h).  no_bitmap: `bitmap` does not hold
+  // the last run's visited states (a checkpoint runs the list layers first).
   CosetMemory* coset = nullptr;
-  bool coset_ok = false, coset_ran = false;
+  RingMemory* ring = nullptr;
+  bool coset_ok = false, ring_ok = false, no_bitmap = false;
+  uint64_t list_stop = 0;  // list layers stop before a layer of this many states (0 = never)
   int coset_run(mgbfs2_status* status);
+  int ring_run(mgbfs2_status* status);
   int run_lists(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, void* user, mgbfs2_status* status);
 
   // Checkpoint / resume (checkpoint.cu): read_checkpoint restores the visited

@@ -1,0 +1,165 @@
+// Whole searches without frontier lists: the handle's side of coset-word
+// layers (coset.h) and scalar-ring layers (ring.h).
+#include <algorithm>
+#include <chrono>
+
+#include "coset.h"
+#include "engine.h"
+#include "ring.h"
+
+namespace mgbfs2 {
+
+#define MG_CHECK(expr)                         \
+  do {                                         \
+    cudaError_t _e = (expr);                   \
+    if (_e != cudaSuccess) return cuda_status(_e); \
+  } while (0)
+
+namespace {
+using Clock = std::chrono::steady_clock;
+
+// List layers until a layer has this share of the ring nodes (below, a
+// layer's pass over every node costs more than its edges), unless there are
+// so few nodes that the pass costs no more than a launch.
+constexpr uint64_t kRingShare = 64, kRingFewNodes = 1ull << 20;
+}  // namespace
+
+// A whole search in coset-word layers, from the identity: the layer sizes do
+// not depend on the start, and its states are those of the identity's search
+// with the codes mapped through the start.
+int Graph::coset_run(mgbfs2_status* status) {
+  mgbfs2_status st{};
+  const auto started = Clock::now();
+  MG_CHECK(cudaEventRecord(ev_run[0], stream));
+  CosetResult r;
+  if (!coset) {
+    coset = new CosetMemory();
+    coset->set_stream(stream);
+  }
+  {
+    TraceRange range("layers.coset");
+    const int rc = coset_wave({CosetJob{elements, gens, perms.data(), inverse_closed}}, kWholeDepth, sm_count, stream,
+                              coset, &r, &front, start_word);
+    if (rc) return rc;
+  }
+  if (r.overflow[0]) {  // deeper than its layer table: the list layers have no such limit
+    return run_lists(nullptr, nullptr, nullptr, status);
+  }
+  no_bitmap = true;
+  front_grouped = false;
+  layer_sizes = r.layers[0];
+  const uint32_t deepest = static_cast<uint32_t>(layer_sizes.size() - 1);
+  layer_seconds.assign(r.step_seconds.begin(), r.step_seconds.begin() + std::min<size_t>(deepest, r.step_seconds.size()));
+  for (int i = 0; i < 2; ++i) {
+    small_layer[i].clear();
+    small_depth[i] = UINT32_MAX;
+  }
+  if (!r.fatal) {
+    if (deepest && layer_sizes[deepest - 1] < kCosetSmall) keep_small(deepest - 1, std::move(r.previous_small));
+    if (layer_sizes[deepest] < kCosetSmall) keep_small(deepest, std::move(r.deepest_small));
+  }
+  last_count = r.fatal ? 0 : layer_sizes[deepest];
+  launches = r.launches;
+  st.complete = r.fatal == 0;
+  st.reason = r.fatal ? MGBFS2_REASON_RESOURCE : MGBFS2_REASON_FRONTIER_EXHAUSTED;
+  st.fatal = r.fatal;
+  st.layers = deepest + 1;
+  for (uint32_t d = 0; d <= deepest; ++d) {
+    const uint64_t c = layer_sizes[d];
+    st.states += c;
+    st.successors += c * gens;
+    st.visited_tests += c * gens - (parent_skip && d > 0 ? c : 0);
+  }
+  if (cudaEventRecord(ev_run[1], stream) == cudaSuccess && cudaEventSynchronize(ev_run[1]) == cudaSuccess) {
+    float ms = 0.f;
+    if (cudaEventElapsedTime(&ms, ev_run[0], ev_run[1]) == cudaSuccess) st.device_seconds = ms * 1e-3;
+  }
+  st.kernel_seconds = r.kernel_seconds;
+  st.bfs_seconds = std::chrono::duration<double>(Clock::now() - started).count();
+  st.kernel_launches = launches;
+  st.peak_device_bytes = std::max<uint64_t>(plan.device_bytes, coset->bytes() + front.bytes);
+  if (status) *status = st;
+  return MGBFS2_OK;
+}
+
+// A search of 2x2 matrices over a prime field: list layers while they are
+// small, then scalar-ring layers to the end.
+int Graph::ring_run(mgbfs2_status* status) {
+  mgbfs2_status st{};
+  const auto started = Clock::now();
+  const uint32_t m = moduli[0];
+  if (ring_nodes(m) > kRingFewNodes) {
+    list_stop = ring_nodes(m) / kRingShare;
+    const int rc = run_lists(nullptr, nullptr, nullptr, &st);
+    list_stop = 0;
+    if (rc || st.reason != MGBFS2_REASON_LAYER_LIMIT) {
+      if (status) *status = st;
+      return rc;
+    }
+  } else {
+    layer_sizes.assign(1, 1);
+    layer_seconds.clear();
+    front_grouped = false;
+    for (int i = 0; i < 2; ++i) {
+      small_layer[i].clear();
+      small_depth[i] = UINT32_MAX;
+    }
+    keep_small(0, std::vector<uint64_t>(1, start_word));
+    last_count = 1;
+    launches = 0;
+    st.states = st.layers = 1;
+    if (int rc = front.ensure(16)) return rc;
+    MG_CHECK(cudaMemcpyAsync(front.ptr, &start_word, 8, cudaMemcpyHostToDevice, stream));
+  }
+  if (!ring) {
+    ring = new RingMemory();
+    ring->set_stream(stream);
+  }
+  std::vector<uint32_t> coef;
+  for (int64_t v : matrices) {
+    v %= static_cast<int64_t>(m);
+    coef.push_back(static_cast<uint32_t>(v < 0 ? v + m : v));
+  }
+  const uint32_t from = static_cast<uint32_t>(layer_sizes.size() - 1);
+  MG_CHECK(cudaEventRecord(ev_run[0], stream));
+  RingResult r;
+  {
+    TraceRange range("layers.ring");
+    const int rc = ring_wave(m, bits, gens, coef.data(), front.ptr, layer_sizes[from], next.ptr,
+                             from ? layer_sizes[from - 1] : 0, key_mask, kWholeDepth, sm_count, stream, ring, &front, &r);
+    if (rc) return rc;
+  }
+  if (r.overflow) return run_lists(nullptr, nullptr, nullptr, status);
+  no_bitmap = true;
+  layer_sizes.insert(layer_sizes.end(), r.layers.begin(), r.layers.end());
+  layer_seconds.insert(layer_seconds.end(), r.seconds.begin(), r.seconds.end());
+  const uint32_t deepest = static_cast<uint32_t>(layer_sizes.size() - 1);
+  if (deepest > from) {
+    if (layer_sizes[deepest - 1] < kRingSmall) keep_small(deepest - 1, std::move(r.previous_small));
+    if (layer_sizes[deepest] < kRingSmall) keep_small(deepest, std::move(r.deepest_small));
+    last_count = layer_sizes[deepest];
+  }
+  launches += r.launches;
+  st.complete = r.fatal == 0;
+  st.reason = r.fatal ? MGBFS2_REASON_RESOURCE : MGBFS2_REASON_FRONTIER_EXHAUSTED;
+  st.fatal = r.fatal;
+  st.layers = deepest + 1;
+  for (uint32_t d = from; d <= deepest; ++d) {
+    const uint64_t c = layer_sizes[d];
+    if (d > from) st.states += c;
+    st.successors += c * gens;
+    st.visited_tests += c * gens - (parent_skip && d > 0 ? c : 0);
+  }
+  if (cudaEventRecord(ev_run[1], stream) == cudaSuccess && cudaEventSynchronize(ev_run[1]) == cudaSuccess) {
+    float ms = 0.f;
+    if (cudaEventElapsedTime(&ms, ev_run[0], ev_run[1]) == cudaSuccess) st.device_seconds += ms * 1e-3;
+  }
+  st.kernel_seconds += r.kernel_seconds;
+  st.bfs_seconds = std::chrono::duration<double>(Clock::now() - started).count();
+  st.kernel_launches = launches;
+  st.peak_device_bytes = std::max<uint64_t>(st.peak_device_bytes, bitmap.bytes + front.bytes + next.bytes + ring->bytes());
+  if (status) *status = st;
+  return MGBFS2_OK;
+}
+
+}  // namespace mgbfs2
