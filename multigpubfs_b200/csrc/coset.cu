@@ -232,35 +232,6 @@ __device__ __forceinline__ unsigned long long decode_state(const RowDecode& r, u
   return w & keep;
 }
 
-// Grid barrier of the cooperative launch: `epoch` counts the barriers passed
-// (the arrival counter only grows).  Bounded like grid_barrier (device.cuh):
-// after kBarrierWaitNs it raises ERR_WAIT_LIMIT and every block ends.
-__device__ __forceinline__ bool coset_barrier(const CosetParams& p, uint32_t* epoch) {
-  __shared__ int ok;
-  __syncthreads();
-  ++*epoch;
-  if (threadIdx.x == 0) {
-    ok = 1;
-    const uint32_t all = *epoch * gridDim.x;
-    uint32_t now;
-    __threadfence();
-    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(now) : "l"(&p.ctl->arrived) : "memory");
-    ++now;
-    const unsigned long long started = global_ns();
-    for (uint32_t polls = 0; static_cast<int32_t>(now - all) < 0; ++polls) {
-      if (polls >= kBarrierPolls || ((polls & 1023u) == 1023u && global_ns() - started > kBarrierWaitNs)) {
-        raise_error(&p.ctl->error, ERR_WAIT_LIMIT);
-        ok = 0;
-        break;
-      }
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&p.ctl->arrived) : "memory");
-    }
-  }
-  __syncthreads();
-  asm volatile("fence.acq_rel.gpu;" ::: "memory");
-  return ok != 0;
-}
-
 // Descriptors of every (row, generator), the slot permutations they need, and
 // the start states.  The parent of a state under g has the label of position p
 // at position g[p].
@@ -470,7 +441,7 @@ __global__ void __launch_bounds__(kCosetBlock, 4) coset_wave_kernel(CosetParams 
   const uint32_t unit_mask = p.units - 1u;
   uint32_t epoch = 0;
   coset_table<W>(p);
-  if (!coset_barrier(p, &epoch)) return;
+  if (!arrival_barrier(&p.ctl->arrived, &p.ctl->error, &epoch)) return;
   CosetInst in = p.inst[0];
   for (uint32_t d = 0;; ++d) {
     if (blockIdx.x == 0 && threadIdx.x == 0) p.stamps[d] = global_ns();
@@ -628,7 +599,7 @@ __global__ void __launch_bounds__(kCosetBlock, 4) coset_wave_kernel(CosetParams 
       }
     }
     if (live) flush();
-    if (!coset_barrier(p, &epoch)) return;
+    if (!arrival_barrier(&p.ctl->arrived, &p.ctl->error, &epoch)) return;
     const bool more = __ldcg(p.active + d + 1) != 0;
     if (more && d < p.max_steps) continue;
     if (blockIdx.x == 0 && threadIdx.x == 0) {

@@ -26,6 +26,7 @@
 #include "coset.h"
 #include "engine.h"
 #include "grouped_kernels.cuh"
+#include "half.h"
 #include "packed_kernels.cuh"
 #include "ring.h"
 
@@ -546,6 +547,11 @@ void Graph::release() {
     ring->release_to_cache(device);
     delete ring;
     ring = nullptr;
+  }
+  if (half) {
+    half->release_to_cache(device);
+    delete half;
+    half = nullptr;
   }
   wide_release();
   if (host_control) {
@@ -1332,6 +1338,19 @@ int Graph::make_plan(const mgbfs2_plan_request* req, mgbfs2_plan_info* out) {
             !r.route_chunk && !r.bucket_min_work && !r.bucket_margin && gens <= kRingMaxGens &&
             (!orbit_bound || orbit_bound >= rank_total) &&
             ring_bytes(moduli[0], kWholeDepth) + bitmap_bytes <= budget / 2;
+  // Permutations with repeated labels in half-rank layers (half.h): packed ones
+  // in place of the fused multinomial bitmap layers, starts of more than 16
+  // positions in place of the wide hash where the bitmap is small and not much
+  // larger than what the generators can reach.
+  const uint64_t reach = state_bound ? std::min(state_bound, rank_total) : rank_total;
+  const HalfJob half_job{elements, distinct, gens, nullptr, nullptr, nullptr, inverse_closed, rank_total, reach};
+  half_ok = kind == 0 && !lehmer && !use_product && r.dedup == MGBFS2_DEDUP_AUTO && !host_loop_only && !r.capacity &&
+            (packed ? visited == MGBFS2_VISITED_BITMAP && bits == 4
+                    : r.visited == MGBFS2_VISITED_AUTO && !r.reserve_bytes && rank_total / 64 <= reach) &&
+            !r.shards && !r.blocks_per_sm && !r.parents_per_thread && !r.route_chunk && !r.bucket_min_work &&
+            !r.bucket_margin && !learned && half_supported(elements, distinct, gens, rank_total) &&
+            (!orbit_bound || orbit_bound >= rank_total) && 16 * (reach + 2) <= (16ull << 30) &&
+            half_bytes(half_job, kWholeDepth) + (rank_total + 63) / 64 * 8 <= budget / 2;
   // Fixed allocations of the plan.
   int rc = MGBFS2_OK;
   if (p.visited == MGBFS2_VISITED_BITMAP && !coset_ok) rc = bitmap.ensure(bitmap_bytes);
@@ -2203,11 +2222,16 @@ int Graph::run(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, void* 
   if (!planned) return MGBFS2_STATE;
   TraceRange range("mgbfs2.run");
   MG_CHECK(cudaSetDevice(device));
-  if (!packed) return wide_run(limits, cb, user, status);
   const bool limited = limits && (limits->max_seconds > 0 || limits->max_layers || limits->cancel);
+  half_done = false;
   if (!limited && !cb && !resume_pending) {
+    if (half_ok) return half_run(status);
     if (coset_ok) return coset_run(status);
     if (ring_ok) return ring_run(status);
+  }
+  if (!packed) {
+    if (half) half->free();
+    return wide_run(limits, cb, user, status);
   }
   return run_lists(limits, cb, user, status);
 }
@@ -2216,6 +2240,7 @@ int Graph::run(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, void* 
 int Graph::run_lists(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, void* user, mgbfs2_status* status) {
   no_bitmap = false;
   if (ring) ring->free();
+  if (half) half->free();
   if (coset_ok) {
     // The plan left the bitmap to the run that needs it, in the place of the
     // coset-word buffers.

@@ -70,6 +70,7 @@ int device_free_bytes(int device, size_t* free_bytes, bool fresh = false);
 struct WideState;     // int64-key arena path (wide.cu)
 struct CosetMemory;   // coset.h
 struct RingMemory;    // ring.h
+struct HalfMemory;    // half.h
 struct ExpandParams;  // packed_kernels.cuh
 
 // A named NVTX range for the lifetime of the object: a profiler's timeline
@@ -197,14 +198,18 @@ struct Graph {
 
   // Searches without frontier lists (whole_search.cu): the default plan of a
   // Lehmer bitmap in coset-word layers (coset.h), of 2x2 matrices over a prime
-  // field in scalar-ring layers (ring.h).  no_bitmap: `bitmap` does not hold
+  // field in scalar-ring layers (ring.h), of repeated labels in half-rank
+  // layers (half.h; half_rows: their samples of wide states).  no_bitmap: `bitmap` does not hold
   // the last run's visited states (a checkpoint runs the list layers first).
   CosetMemory* coset = nullptr;
   RingMemory* ring = nullptr;
-  bool coset_ok = false, ring_ok = false, no_bitmap = false;
+  HalfMemory* half = nullptr;
+  bool coset_ok = false, ring_ok = false, half_ok = false, no_bitmap = false, half_done = false;
+  std::vector<std::vector<int64_t>> half_rows[2];
   uint64_t list_stop = 0;  // list layers stop before a layer of this many states (0 = never)
   int coset_run(mgbfs2_status* status);
   int ring_run(mgbfs2_status* status);
+  int half_run(mgbfs2_status* status);
   int run_lists(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, void* user, mgbfs2_status* status);
 
   // Checkpoint / resume (checkpoint.cu): read_checkpoint restores the visited

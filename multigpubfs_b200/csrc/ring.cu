@@ -192,32 +192,6 @@ __device__ __forceinline__ void or_rotated(uint32_t (&acc)[NW], const uint32_t (
     acc[i] |= __funnelshift_r(y[i], y[i + 1], s & 31u) | __funnelshift_l(z[i], z[i + 1], n & 31u);
 }
 
-__device__ __forceinline__ bool ring_barrier(const RingParams& r, uint32_t* epoch) {
-  __shared__ int ok;
-  __syncthreads();
-  ++*epoch;
-  if (threadIdx.x == 0) {
-    ok = 1;
-    const uint32_t all = *epoch * gridDim.x;
-    uint32_t now;
-    __threadfence();
-    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(now) : "l"(&r.ctl->arrived) : "memory");
-    ++now;
-    const unsigned long long started = global_ns();
-    for (uint32_t polls = 0; static_cast<int32_t>(now - all) < 0; ++polls) {
-      if (polls >= kBarrierPolls || ((polls & 1023u) == 1023u && global_ns() - started > kBarrierWaitNs)) {
-        raise_error(&r.ctl->error, ERR_WAIT_LIMIT);
-        ok = 0;
-        break;
-      }
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&r.ctl->arrived) : "memory");
-    }
-  }
-  __syncthreads();
-  asm volatile("fence.acq_rel.gpu;" ::: "memory");
-  return ok != 0;
-}
-
 // The states of layer d (from the seeded one) as packed words, and block 0's report.
 template <int NW>
 __device__ void ring_finish(const RingParams& r, const Tables& t, uint32_t d, bool exhausted) {
@@ -317,7 +291,7 @@ __global__ void __launch_bounds__(kRingBlock, 4) ring_wave_kernel(RingParams r) 
     }
     found = __reduce_add_sync(kFullMask, found);
     if (found && (threadIdx.x & 31u) == 0) atomicAdd(r.counts + d + 1, static_cast<unsigned long long>(found));
-    if (!ring_barrier(r, &epoch)) return;
+    if (!arrival_barrier(&r.ctl->arrived, &r.ctl->error, &epoch)) return;
     const bool more = __ldcg(r.counts + d + 1) != 0;
     if (more && d < r.max_steps) continue;
     if (blockIdx.x == 0) {

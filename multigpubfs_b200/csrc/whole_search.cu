@@ -1,10 +1,11 @@
 // Whole searches without frontier lists: the handle's side of coset-word
-// layers (coset.h) and scalar-ring layers (ring.h).
+// layers (coset.h), scalar-ring layers (ring.h) and half-rank layers (half.h).
 #include <algorithm>
 #include <chrono>
 
 #include "coset.h"
 #include "engine.h"
+#include "half.h"
 #include "ring.h"
 
 namespace mgbfs2 {
@@ -158,6 +159,83 @@ int Graph::ring_run(mgbfs2_status* status) {
   st.bfs_seconds = std::chrono::duration<double>(Clock::now() - started).count();
   st.kernel_launches = launches;
   st.peak_device_bytes = std::max<uint64_t>(st.peak_device_bytes, bitmap.bytes + front.bytes + next.bytes + ring->bytes());
+  if (status) *status = st;
+  return MGBFS2_OK;
+}
+
+// A search over repeated labels in half-rank layers, packed or wide.
+int Graph::half_run(mgbfs2_status* status) {
+  mgbfs2_status st{};
+  const auto started = Clock::now();
+  if (!half) {
+    half = new HalfMemory();
+    half->set_stream(stream);
+  }
+  const uint64_t reach = state_bound ? std::min(state_bound, rank_total) : rank_total;
+  const HalfJob job{elements, distinct, gens, codes.data(), code_counts.data(), perms.data(), inverse_closed, rank_total, reach};
+  MG_CHECK(cudaEventRecord(ev_run[0], stream));
+  HalfResult r;
+  {
+    TraceRange range("layers.half");
+    const int rc = half_wave(job, kWholeDepth, sm_count, stream, half, &bitmap, packed ? &front : nullptr, bits, &r);
+    if (rc) return rc;
+  }
+  if (r.overflow) return packed ? run_lists(nullptr, nullptr, nullptr, status) : wide_run(nullptr, nullptr, nullptr, status);
+  no_bitmap = false;  // the bitmap over the rank domain is the one list layers make
+  front_grouped = false;
+  layer_sizes = r.layers;
+  layer_seconds = r.seconds;
+  const uint32_t deepest = static_cast<uint32_t>(layer_sizes.size() - 1);
+  for (int i = 0; i < 2; ++i) {
+    small_layer[i].clear();
+    small_depth[i] = UINT32_MAX;
+    half_rows[i].clear();
+  }
+  const auto symbol = [&](uint64_t w, uint32_t i) { return (w >> (r.bits * i)) & ((1ull << r.bits) - 1ull); };
+  if (packed) {
+    const auto words = [&](const std::vector<uint64_t>& states) {
+      std::vector<uint64_t> out;
+      for (uint64_t w : states) {
+        uint64_t v = 0;
+        for (uint32_t i = 0; i < elements; ++i) v |= symbol(w, i) << (bits * i);
+        out.push_back(v);
+      }
+      return out;
+    };
+    if (deepest && layer_sizes[deepest - 1] < kHalfSmall) keep_small(deepest - 1, words(r.previous));
+    if (layer_sizes[deepest] < kHalfSmall) keep_small(deepest, words(r.deepest));
+  } else {
+    half_done = true;
+    const auto rows = [&](const std::vector<uint64_t>& states, std::vector<std::vector<int64_t>>* out) {
+      for (uint64_t w : states) {
+        std::vector<int64_t> row(elements);
+        for (uint32_t i = 0; i < elements; ++i) row[i] = labels[symbol(w, i)];
+        out->push_back(std::move(row));
+      }
+    };
+    rows(r.deepest, &half_rows[0]);
+    rows(r.previous, &half_rows[1]);
+  }
+  last_count = r.fatal ? 0 : layer_sizes[deepest];
+  launches = r.launches;
+  st.complete = r.fatal == 0;
+  st.reason = r.fatal ? MGBFS2_REASON_RESOURCE : MGBFS2_REASON_FRONTIER_EXHAUSTED;
+  st.fatal = r.fatal;
+  st.layers = deepest + 1;
+  for (uint32_t d = 0; d <= deepest; ++d) {
+    const uint64_t c = layer_sizes[d];
+    st.states += c;
+    st.successors += c * gens;
+    if (packed) st.visited_tests += c * gens - (parent_skip && d > 0 ? c : 0);
+  }
+  if (cudaEventRecord(ev_run[1], stream) == cudaSuccess && cudaEventSynchronize(ev_run[1]) == cudaSuccess) {
+    float ms = 0.f;
+    if (cudaEventElapsedTime(&ms, ev_run[0], ev_run[1]) == cudaSuccess) st.device_seconds = ms * 1e-3;
+  }
+  st.kernel_seconds = r.kernel_seconds;
+  st.bfs_seconds = std::chrono::duration<double>(Clock::now() - started).count();
+  st.kernel_launches = launches;
+  st.peak_device_bytes = std::max<uint64_t>(plan.device_bytes, bitmap.bytes + front.bytes + half->bytes());
   if (status) *status = st;
   return MGBFS2_OK;
 }

@@ -373,6 +373,16 @@ int Graph::wide_run(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, v
 }
 
 int Graph::wide_sample(uint32_t which, int64_t* out, size_t cap_rows, size_t* rows) {
+  if (half_done) {  // the last run was in half-rank layers: their rows are kept on the host
+    const auto& kept = half_rows[which];
+    const uint64_t n = std::min<uint64_t>(kept.size(), cap_rows);
+    std::vector<std::vector<int64_t>> sorted(kept.begin(), kept.begin() + static_cast<std::ptrdiff_t>(n));
+    std::sort(sorted.begin(), sorted.end());
+    for (uint64_t r = 0; r < n; ++r)
+      if (out) std::memcpy(out + r * elements, sorted[r].data(), elements * sizeof(int64_t));
+    *rows = n;
+    return MGBFS2_OK;
+  }
   WideState& w = *wide;
   uint64_t begin = w.last_begin, count = w.last_count;
   if (which == 1) {

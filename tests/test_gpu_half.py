@@ -1,0 +1,90 @@
+"""Half-rank layers (repeated labels under the default plan) against the oracle
+and the list layers: one to six labels, odd and even degrees, both sides of the
+limits that send a start to the general paths, directed sets and the wide
+starts of more than 16 positions."""
+import random
+
+import pytest
+
+from oracle import graph_oracle as G
+from oracle import packed_oracle as P
+
+pytestmark = pytest.mark.gpu
+
+
+def _search(graph, **plan):
+    from multigpubfs_b200 import GraphDefinition
+    from multigpubfs_b200.engine import NativeGraph
+    with NativeGraph(GraphDefinition.from_dict(graph)) as e:
+        info = e.plan(**plan)
+        r = e.run()
+        words = sorted(e.frontier_words().tolist()) if info["packed"] else None
+        return r, e.sample(0, 1000), e.sample(1, 1000), words
+
+
+def _start(rng, n, labels):
+    names = rng.sample(range(-50, 50), labels)
+    start = [names[i % labels] for i in range(n)]
+    rng.shuffle(start)
+    return start
+
+
+@pytest.mark.parametrize("n", [2, 3, 7, 8, 9, 13, 15, 16])
+@pytest.mark.parametrize("labels", [1, 2, 3, 4, 5, 6, 7])
+def test_packed_starts(n, labels):
+    if labels >= n or (n > 13 and labels > 4):
+        pytest.skip("distinct labels, or a domain past a quick comparison")
+    rng = random.Random(100 * n + labels)
+    closed = labels % 2 == 0
+    gens = G.lrx_generators(n) if closed else [rng.sample(range(n), n) for _ in range(3)]
+    graph = G.permutation_graph(gens, _start(rng, n, labels))
+    lists, last, small, words = _search(graph, visited="bitmap", dedup="atomic")
+    r, current, previous, front = _search(graph)
+    assert r.layer_sizes == lists.layer_sizes
+    assert (r.states, r.successors, r.visited_tests) == (lists.states, lists.successors, lists.visited_tests)
+    assert previous == small and front == words
+    if r.layer_sizes[-1] <= 1000:
+        assert current == last
+    if n <= 9:
+        assert r.layer_sizes == P.packed_bfs(gens, graph["start"])[0]
+
+
+@pytest.mark.parametrize("n,labels", [(17, 1), (17, 2), (18, 2), (17, 3), (17, 4), (17, 5), (24, 2), (37, 2)])
+@pytest.mark.parametrize("closed", [True, False])
+def test_wide_starts(n, labels, closed):
+    """More than 16 positions, against the wide hash (visited="hash" asks for
+    it); 17 positions of five labels and 37 of two keep the hash by default."""
+    rng = random.Random(10 * n + labels)
+    start = [0] * (n - 3) + [1, 1, 2][:3] if n == 37 else _start(rng, n, labels)
+    if n == 37:
+        start = [min(x, 1) for x in start]
+    gens = G.lrx_generators(n) if closed else G.lrx_generators(n)[::2]
+    if labels == 5:
+        start = [0] * (n - 4) + [1, 2, 3, 4]
+    graph = G.permutation_graph(gens, start)
+    lists, last, small, _ = _search(graph, visited="hash")
+    r, current, previous, _ = _search(graph)
+    assert r.complete and r.layer_sizes == lists.layer_sizes
+    assert (r.states, r.successors, r.visited_tests) == (lists.states, lists.successors, lists.visited_tests)
+    assert previous == small
+    if r.layer_sizes[-1] <= 1000:
+        assert current == last
+
+
+def test_the_bitmap_is_the_list_layers(tmp_path):
+    """A checkpoint of a finished search loads, and one of list layers goes on
+    to the same table."""
+    from multigpubfs_b200 import GraphDefinition
+    from multigpubfs_b200.engine import NativeGraph
+    g = GraphDefinition.from_dict(G.permutation_graph(G.lrx_generators(12), [i % 4 for i in range(12)]))
+    with NativeGraph(g) as e:
+        e.plan()
+        full = e.run()
+        e.checkpoint(tmp_path / "done.bin")
+        e.run(max_layers=9)
+        e.checkpoint(tmp_path / "part.bin")
+    for name in ("done.bin", "part.bin"):
+        with NativeGraph(g) as e:
+            e.plan()
+            e.resume(tmp_path / name)
+            assert e.run().layer_sizes == full.layer_sizes
