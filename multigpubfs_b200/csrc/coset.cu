@@ -17,6 +17,7 @@ namespace {
 constexpr uint32_t kSlots = 7, kSlotPerms = 5040;
 constexpr uint32_t kCosetBlock = 256, kCosetWarps = kCosetBlock / 32;
 constexpr uint32_t kMaxUnits = 8;  // units (128 nodes) of a work item
+constexpr size_t kSmallMaxShared = 160 << 10;  // parent words of a block of the small kernel
 
 struct CosetInst {
   uint32_t m, gens, rows, inverse_closed;
@@ -232,6 +233,61 @@ __device__ __forceinline__ unsigned long long decode_state(const RowDecode& r, u
   return w & keep;
 }
 
+// tau, four bits a slot, from its Lehmer code.
+__device__ __forceinline__ uint32_t slot_permutation(uint32_t code) {
+  uint32_t digits = 0, tau = 0, seen = 0;
+#pragma unroll
+  for (uint32_t a = kSlots; a-- > 0;) {
+    digits |= (code % (kSlots - a)) << (4 * a);
+    code /= kSlots - a;
+  }
+  for (uint32_t a = 0; a < kSlots; ++a) {
+    const uint32_t to = nth_free(seen, (digits >> (4 * a)) & 15u);
+    tau |= to << (4 * a);
+    seen |= 1u << to;
+  }
+  return tau;
+}
+
+// Image of a node under a slot permutation, and the inner flips.
+__device__ __forceinline__ uint32_t node_image(uint32_t tau, uint32_t x, uint32_t* flips) {
+  const uint32_t slots = kNodeSlots.at[x];
+  uint32_t used = 0, to = 0, f = 0;
+#pragma unroll
+  for (uint32_t t = 0; t < 3; ++t) {
+    const uint32_t a = (tau >> (4 * ((slots >> (8 * t)) & 15u))) & 15u;
+    const uint32_t b = (tau >> (4 * ((slots >> (8 * t + 4)) & 15u))) & 15u;
+    const uint32_t lo = min(a, b), hi = max(a, b), c = 7 - 2 * t;
+    const uint32_t i = lo - bits_below(used, lo), j = hi - bits_below(used, hi);
+    f |= (a > b ? 1u : 0u) << t;
+    to = to * (c * (c - 1) / 2) + j * (j - 1) / 2 + i;
+    used |= (1u << a) | (1u << b);
+  }
+  *flips = f;
+  return to;
+}
+
+// Parent row of a row under a generator (position images `perm`), the slot
+// permutation's Lehmer code and the outer flips.
+__device__ __forceinline__ uint32_t row_image(uint32_t m, uint32_t row, const uint8_t* perm, uint32_t* code,
+                                              uint32_t* flips) {
+  uint8_t pos[7], image[7];
+  const uint32_t used = row_positions(m, row, pos);
+  for (uint32_t l = 0; l < m - kSlots; ++l) image[l] = perm[pos[l]];
+  uint32_t mask;
+  const uint32_t parent = row_rank(m, image, flips, &mask);
+  // Slot a of the row goes to slot tau[a] of the parent row.
+  uint32_t c = 0, seen = 0, at = 0;
+  for (uint32_t a = 0; a < kSlots; ++a, ++at) {
+    while ((used >> at) & 1u) ++at;
+    const uint32_t image_at = perm[at], tau = image_at - bits_below(mask, image_at);
+    c = c * (kSlots - a) + tau - bits_below(seen, tau);
+    seen |= 1u << tau;
+  }
+  *code = c;
+  return parent;
+}
+
 // Descriptors of every (row, generator), the slot permutations they need, and
 // the start states.  The parent of a state under g has the label of position p
 // at position g[p].
@@ -248,20 +304,8 @@ __global__ void __launch_bounds__(kCosetBlock) coset_setup(CosetParams p) {
     }
     const CosetInst in = p.inst[lo];
     const uint32_t local = static_cast<uint32_t>(t - in.desc_off), row = local / in.gens, g = local % in.gens;
-    const uint8_t* perm = p.perms + in.perm_off + 16 * g;
-    uint8_t pos[7], image[7];
-    const uint32_t used = row_positions(in.m, row, pos);
-    for (uint32_t l = 0; l < in.m - kSlots; ++l) image[l] = perm[pos[l]];
-    uint32_t flips, mask;
-    const uint32_t parent = row_rank(in.m, image, &flips, &mask);
-    // Slot a of the row goes to slot tau[a] of the parent row.
-    uint32_t code = 0, seen = 0, at = 0;
-    for (uint32_t a = 0; a < kSlots; ++a, ++at) {
-      while ((used >> at) & 1u) ++at;
-      const uint32_t image_at = perm[at], tau = image_at - bits_below(mask, image_at);
-      code = code * (kSlots - a) + tau - bits_below(seen, tau);
-      seen |= 1u << tau;
-    }
+    uint32_t code, flips;
+    const uint32_t parent = row_image(in.m, row, p.perms + in.perm_off + 16 * g, &code, &flips);
     p.used[code] = 1;
     p.desc[t] = parent | (static_cast<unsigned long long>(code) << 32) | (static_cast<unsigned long long>(flips) << 48);
   }
@@ -302,33 +346,12 @@ __device__ void coset_table(const CosetParams& p) {
     uint32_t found = __ballot_sync(kFullMask, mine < kSlotPerms && __ldcg(p.used + mine));
     for (; found; found &= found - 1) {
       const uint32_t perm = (base + __ffs(static_cast<int>(found)) - 1) * warps + warp;
-      // tau, four bits a slot, from its Lehmer code.
-      uint32_t code = perm, digits = 0, tau = 0, seen = 0;
-#pragma unroll
-      for (uint32_t a = kSlots; a-- > 0;) {
-        digits |= (code % (kSlots - a)) << (4 * a);
-        code /= kSlots - a;
-      }
-      for (uint32_t a = 0; a < kSlots; ++a) {
-        const uint32_t to = nth_free(seen, (digits >> (4 * a)) & 15u);
-        tau |= to << (4 * a);
-        seen |= 1u << to;
-      }
+      const uint32_t tau = slot_permutation(perm);
       for (uint32_t x = lane; x < kCosetStride; x += 32) {
         uint32_t out = table_entry<W>(x, 0);  // words past the nodes stay zero and map to themselves
         if (x < kCosetNodes) {
-          const uint32_t slots = kNodeSlots.at[x];
-          uint32_t used = 0, to = 0, flips = 0;
-#pragma unroll
-          for (uint32_t t = 0; t < 3; ++t) {
-            const uint32_t a = (tau >> (4 * ((slots >> (8 * t)) & 15u))) & 15u;
-            const uint32_t b = (tau >> (4 * ((slots >> (8 * t + 4)) & 15u))) & 15u;
-            const uint32_t lo = min(a, b), hi = max(a, b), c = 7 - 2 * t;
-            const uint32_t i = lo - bits_below(used, lo), j = hi - bits_below(used, hi);
-            flips |= (a > b ? 1u : 0u) << t;
-            to = to * (c * (c - 1) / 2) + j * (j - 1) / 2 + i;
-            used |= (1u << a) | (1u << b);
-          }
+          uint32_t flips;
+          const uint32_t to = node_image(tau, x, &flips);
           out = table_entry<W>(to, flips);
         }
         p.table[perm * kCosetStride + x] = out;
@@ -618,6 +641,213 @@ __global__ void __launch_bounds__(kCosetBlock) coset_collect(CosetParams p, uint
   coset_finish<W>(p, p.inst[0], last, true);
 }
 
+// Small searches: every unit (128 nodes) has a warp of its own for the whole
+// search, which keeps its words of layers d and d - 1 (and of the visited set)
+// in registers and the address and flips of every parent word in shared memory.
+// A layer is then one gather from L2 per generator, one store and one barrier;
+// the general kernel's chain of dependent L2 reads (items, descriptors, flags,
+// table, words) took 5.5 us a layer on S8 and 9 us on S10 with nothing to
+// read.  No tables are made: the descriptors are computed where they are used.
+struct SmallParams {
+  uint32_t n, m, gens, units, inverse_closed, max_steps;
+  uint8_t perms[kCosetMaxGens * 16];
+  uint32_t* buf[2];
+  unsigned long long* counts;
+  unsigned long long* stamps;
+  // Barrier and layer size in one: arrivals in the low half, states found so
+  // far in the high half (a search of up to 10! states).
+  unsigned long long* arrived;
+  CosetCtl* ctl;
+  uint32_t* small_count;
+  unsigned long long* small;  // kCosetSmall entries (node word * 64 + bit) of the last small layer overwritten, by parity
+  CosetReport* report;
+  unsigned long long* front;
+  unsigned long long front_cap, start;
+};
+
+// Parent word of a node: index in the buffer, outer flips in bits 24..25, the
+// inner nibble shift (0 or 4) in bits 26..28, the byte flips in bits 30..31.
+constexpr uint32_t kSmallIndexMask = (1u << 24) - 1u;
+
+__device__ __forceinline__ uint32_t flip_small(uint32_t w, uint32_t e) {
+  w = __byte_perm(w, 0u, 0x3210u ^ ((e >> 30) * 0x1111u));
+  const uint32_t by = (e >> 26) & 7u;
+  w = ((w << by) & 0xf0f0f0f0u) | ((w >> by) & 0x0f0f0f0fu);
+  return flip_outer(w, (e >> 24) & 3u);
+}
+
+__device__ __forceinline__ void small_states(const SmallParams& p, uint32_t unit, uint32_t lane, const uint32_t (&w)[4]) {
+  const unsigned long long keep = (1ull << (4 * p.n)) - 1ull;
+  const uint32_t row = unit / kCosetParts, x0 = (unit - row * kCosetParts) * 128u + lane;
+  if (!(w[0] | w[1] | w[2] | w[3])) return;
+  const RowDecode dec = decode_row(p.m, row, p.start);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (!w[k]) continue;
+    unsigned long long at = atomicAdd(&p.ctl->collected, static_cast<unsigned long long>(__popc(w[k])));
+    for (uint32_t b = w[k]; b; b &= b - 1, ++at) {
+      const unsigned long long s = decode_state<false>(dec, x0 + 32 * k, lowest_bit(b), p.start, keep);
+      if (at < p.front_cap) p.front[at] = s;
+      if (at < kCosetSmall) p.report->deepest[at] = s;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kCosetBlock, 4) coset_small_kernel(SmallParams p) {
+  extern __shared__ uint32_t parents[];  // warp x generator x 128 nodes
+  __shared__ uint32_t sums[kCosetWarps];
+  __shared__ unsigned long long seen;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t unit = blockIdx.x * kCosetWarps + warp;
+  const bool mine = unit < p.units;
+  const uint32_t row = unit / kCosetParts, x0 = (unit - row * kCosetParts) * 128u + lane;
+  const size_t own = static_cast<size_t>(row) * kCosetStride + x0;
+  uint32_t* from = parents + warp * p.gens * 128u + lane;
+  uint32_t a[4] = {0, 0, 0, 0}, b[4] = {0, 0, 0, 0}, v[4] = {0, 0, 0, 0};  // layers d and d - 1, visited
+  if (mine) {
+    uint32_t parent = 0, tau = 0, q = 0;
+    if (lane < p.gens) {
+      uint32_t code;
+      parent = row_image(p.m, row, p.perms + 16 * lane, &code, &q);
+      tau = slot_permutation(code);
+    }
+    for (uint32_t g = 0; g < p.gens; ++g) {
+      const uint32_t row_g = __shfl_sync(kFullMask, parent, g), tau_g = __shfl_sync(kFullMask, tau, g);
+      const uint32_t q_g = __shfl_sync(kFullMask, q, g);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t x = x0 + 32 * k;
+        uint32_t flips = 0;
+        const uint32_t to = x < kCosetNodes ? node_image(tau_g, x, &flips) : x;
+        from[g * 128u + 32 * k] =
+            (row_g * kCosetStride + to) | (q_g << 24) | ((flips & 1u) << 28) | ((flips >> 1) << 30);
+      }
+    }
+    // The identity: outer label l at position l, node 0, no flips.
+    uint8_t pos[7];
+    for (uint32_t l = 0; l < kSlots; ++l) pos[l] = static_cast<uint8_t>(kSlots + l);
+    uint32_t f, mask;
+    if (row == row_rank(p.m, pos, &f, &mask) && x0 == 0) a[0] = v[0] = 1;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      p.buf[0][own + 32 * k] = a[k];
+      p.buf[1][own + 32 * k] = 0;
+    }
+  }
+  uint32_t epoch = 0;
+  // Ends the block's part of a layer that found `found` states in this thread;
+  // returns the states found so far by all, or ~0 when the wait gave up.
+  const auto arrive = [&](uint32_t found) {
+    const uint32_t sum = __reduce_add_sync(kFullMask, found);
+    if (lane == 0) sums[warp] = sum;
+    __syncthreads();
+    ++epoch;
+    if (threadIdx.x == 0) {
+      unsigned long long add = 0, now;
+      for (uint32_t w = 0; w < kCosetWarps; ++w) add += sums[w];
+      add = (add << 32) | 1ull;
+      const uint32_t all = epoch * gridDim.x;
+      __threadfence();
+      asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;" : "=l"(now) : "l"(p.arrived), "l"(add) : "memory");
+      now += add;
+      const unsigned long long started = global_ns();
+      for (uint32_t polls = 0; static_cast<int32_t>(static_cast<uint32_t>(now) - all) < 0; ++polls) {
+        if (polls >= kBarrierPolls || ((polls & 1023u) == 1023u && global_ns() - started > kBarrierWaitNs)) {
+          raise_error(&p.ctl->error, ERR_WAIT_LIMIT);
+          now = ~0ull;
+          break;
+        }
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(p.arrived) : "memory");
+      }
+      seen = now;
+    }
+    __syncthreads();
+    const unsigned long long all_found = seen;
+    return all_found == ~0ull ? all_found : all_found >> 32;
+  };
+  unsigned long long total = 0;
+  if (arrive(0) == ~0ull) return;
+  unsigned long long size = 1, before = ~0ull;  // layers d and d - 1
+  for (uint32_t d = 0;; ++d) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      p.stamps[d] = global_ns();
+      p.counts[d] = size;
+    }
+    uint32_t found = 0;
+    if (mine) {
+      const uint32_t* cur = p.buf[d & 1u];
+      uint32_t acc[4] = {0, 0, 0, 0};
+      // Read past L1, which may hold words of two layers ago.
+#pragma unroll 2
+      for (uint32_t g = 0; g < p.gens; ++g) {
+        uint32_t e[4], w[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) e[k] = from[g * 128u + 32 * k];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) w[k] = __ldcg(cur + (e[k] & kSmallIndexMask));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[k] |= flip_small(w[k], e[k]);
+      }
+      uint32_t* nxt = p.buf[(d & 1u) ^ 1u] + own;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        acc[k] &= p.inverse_closed ? ~(a[k] | b[k]) : ~v[k];
+        v[k] |= acc[k];
+        found += __popc(acc[k]);
+        if (acc[k] != b[k]) nxt[32 * k] = acc[k];
+        if (before < kCosetSmall)
+          for (uint32_t o = b[k]; o; o &= o - 1) {
+            const uint32_t at = atomicAdd(p.small_count + d, 1u);
+            if (at < kCosetSmall) p.small[(d & 1u) * kCosetSmall + at] = (own + 32 * k) * 64ull + lowest_bit(o);
+          }
+        b[k] = a[k];
+        a[k] = acc[k];
+      }
+    }
+    const unsigned long long now = arrive(found);
+    if (now == ~0ull) return;
+    before = size;
+    size = now - total;
+    total = now;
+    if (size && d < p.max_steps) continue;
+    // b holds layer d, the deepest when nothing was found.
+    if (!size && mine && before <= p.front_cap) small_states(p, unit, lane, b);
+    if (blockIdx.x) return;
+    const uint32_t kept = size ? 0u : min(__ldcg(p.small_count + d), kCosetSmall);
+    const unsigned long long keep = (1ull << (4 * p.n)) - 1ull;
+    for (uint32_t k = threadIdx.x; k < kept; k += blockDim.x) {
+      const unsigned long long at = __ldcg(p.small + (d & 1u) * kCosetSmall + k), w = at / 64;
+      const RowDecode dec = decode_row(p.m, static_cast<uint32_t>(w / kCosetStride), p.start);
+      p.report->previous[k] = decode_state<false>(dec, static_cast<uint32_t>(w % kCosetStride),
+                                                  static_cast<uint32_t>(at % 64), p.start, keep);
+    }
+    if (threadIdx.x == 0) {
+      p.counts[d + 1] = size;
+      p.stamps[d + 1] = global_ns();
+      p.ctl->steps = d + 1;
+      p.report->previous_count = kept;
+      p.report->steps = d + 1;
+      p.report->error = p.ctl->error;
+    }
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < kReportLayers && k <= d + 1; k += blockDim.x) {
+      p.report->counts[k] = p.counts[k];
+      p.report->stamps[k] = p.stamps[k];
+    }
+    return;
+  }
+}
+
+// The deepest layer of a small search again, into a buffer that holds it.
+__global__ void __launch_bounds__(kCosetBlock) coset_small_collect(SmallParams p, uint32_t last) {
+  const uint32_t lane = threadIdx.x & 31u, unit = blockIdx.x * kCosetWarps + (threadIdx.x >> 5);
+  if (unit >= p.units) return;
+  const uint32_t row = unit / kCosetParts, x0 = (unit - row * kCosetParts) * 128u + lane;
+  const uint32_t* words = p.buf[last & 1u] + static_cast<size_t>(row) * kCosetStride + x0;
+  const uint32_t w[4] = {words[0], words[32], words[64], words[96]};
+  small_states(p, unit, lane, w);
+}
+
 size_t al256(size_t x) { return (x + 255) / 256 * 256; }
 
 uint32_t embedded(uint32_t n) { return std::max(n, kSlots); }
@@ -641,6 +871,101 @@ uint64_t coset_fixed_bytes(uint32_t max_depth) {
   return table_bytes() + kSlotPerms + 16ull * kCosetSmall + 20ull * (max_depth + 2) + 32 * 256;
 }
 
+// Layer tables (count x cols sizes, 0 past the deepest) and step times.
+static void read_layers(const std::vector<unsigned long long>& counts, const std::vector<unsigned long long>& stamps,
+                        uint32_t count, uint32_t cols, uint32_t max_depth, CosetResult* out) {
+  out->layers.assign(count, {});
+  out->overflow.assign(count, 0);
+  for (uint32_t i = 0; i < count; ++i) {
+    const unsigned long long* row = counts.data() + static_cast<size_t>(i) * cols;
+    for (uint32_t d = 0; d < cols && row[d]; ++d) out->layers[i].push_back(row[d]);
+    out->overflow[i] = out->layers[i].size() > max_depth;
+  }
+  out->step_seconds.clear();
+  for (uint32_t d = 0; d + 1 < cols; ++d) out->step_seconds.push_back(static_cast<double>(stamps[d + 1] - stamps[d]) * 1e-9);
+  out->kernel_seconds = cols > 1 ? static_cast<double>(stamps[cols - 1] - stamps[0]) * 1e-9 : 0.0;
+}
+
+// One job through the small kernel: one clear, one launch, one synchronisation.
+static int coset_small(const CosetJob& job, uint32_t max_depth, uint32_t units, size_t smem, cudaStream_t stream,
+                       CosetMemory* memory, CosetResult* out, DeviceBuffer* collect, uint64_t start_word) {
+  SmallParams p{};
+  p.n = job.n;
+  p.m = embedded(job.n);
+  p.gens = job.gens;
+  p.units = units;
+  p.inverse_closed = job.inverse_closed;
+  p.max_steps = max_depth - 1;
+  p.start = start_word;
+  for (uint32_t g = 0; g < job.gens; ++g)
+    for (uint32_t k = 0; k < 16; ++k)
+      p.perms[16 * g + k] = static_cast<uint8_t>(k < job.n ? job.perms[static_cast<size_t>(g) * job.n + k] : k);
+  const uint32_t stride = max_depth + 2;
+  size_t off = 0;
+  const auto take = [&off](size_t bytes) {
+    const size_t at = off;
+    off = al256(off + bytes);
+    return at;
+  };
+  const size_t o_ctl = take(sizeof(CosetCtl)), o_arrived = take(8), o_small_count = take(4ull * stride);
+  const size_t cleared = off;
+  const size_t o_counts = take(8ull * stride), o_stamps = take(8ull * stride), o_small = take(16ull * kCosetSmall);
+  const size_t words = static_cast<size_t>(units) * 128 * sizeof(uint32_t);
+  const size_t o_buf0 = take(words), o_buf1 = take(words);
+  int rc = memory->arena.ensure(off, true);
+  if (!rc) rc = collect->ensure((kCosetSmall + 2) * 8);
+  if (!rc && !memory->report) rc = pinned_take(sizeof(CosetReport), &memory->report);
+  if (rc) return rc;
+  char* base = static_cast<char*>(memory->arena.ptr);
+  p.ctl = reinterpret_cast<CosetCtl*>(base + o_ctl);
+  p.arrived = reinterpret_cast<unsigned long long*>(base + o_arrived);
+  p.small_count = reinterpret_cast<uint32_t*>(base + o_small_count);
+  p.counts = reinterpret_cast<unsigned long long*>(base + o_counts);
+  p.stamps = reinterpret_cast<unsigned long long*>(base + o_stamps);
+  p.small = reinterpret_cast<unsigned long long*>(base + o_small);
+  p.buf[0] = reinterpret_cast<uint32_t*>(base + o_buf0);
+  p.buf[1] = reinterpret_cast<uint32_t*>(base + o_buf1);
+  p.report = static_cast<CosetReport*>(memory->report);
+  p.report->steps = 0;
+  p.front = static_cast<unsigned long long*>(collect->ptr);
+  p.front_cap = collect->bytes / 8;
+  const uint32_t blocks = (units + kCosetWarps - 1) / kCosetWarps;
+  void* args[] = {&p};
+  MG_CHECK_COSET(cudaMemsetAsync(base, 0, cleared, stream));
+  MG_CHECK_COSET(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(coset_small_kernel), dim3(blocks),
+                                             dim3(kCosetBlock), args, smem, stream));
+  MG_CHECK_COSET(cudaStreamSynchronize(stream));
+  out->launches = 1;
+  out->steps = p.report->steps;
+  out->fatal = out->steps ? p.report->error : static_cast<uint32_t>(ERR_WAIT_LIMIT);  // no report: a barrier gave up
+  const uint32_t cols = std::min(out->steps + 1, stride);
+  std::vector<unsigned long long> counts(cols, 0), stamps(cols, 0);
+  if (cols <= kReportLayers) {
+    std::memcpy(counts.data(), p.report->counts, 8ull * cols);
+    std::memcpy(stamps.data(), p.report->stamps, 8ull * cols);
+  } else {
+    MG_CHECK_COSET(cudaMemcpyAsync(counts.data(), p.counts, 8ull * cols, cudaMemcpyDeviceToHost, stream));
+    MG_CHECK_COSET(cudaMemcpyAsync(stamps.data(), p.stamps, 8ull * cols, cudaMemcpyDeviceToHost, stream));
+    MG_CHECK_COSET(cudaStreamSynchronize(stream));
+  }
+  if (out->fatal) counts.assign(1, 1);
+  read_layers(counts, stamps, 1, static_cast<uint32_t>(counts.size()), max_depth, out);
+  if (out->fatal || out->overflow[0]) return MGBFS2_OK;
+  out->previous_small.assign(p.report->previous, p.report->previous + p.report->previous_count);
+  const uint64_t deepest = out->layers[0].back();
+  if (deepest <= kCosetSmall) out->deepest_small.assign(p.report->deepest, p.report->deepest + deepest);
+  if (deepest <= p.front_cap) return MGBFS2_OK;
+  if ((rc = collect->ensure((deepest + 2) * 8))) return rc;
+  p.front = static_cast<unsigned long long*>(collect->ptr);
+  p.front_cap = deepest;
+  MG_CHECK_COSET(cudaMemsetAsync(&p.ctl->collected, 0, sizeof(unsigned long long), stream));
+  coset_small_collect<<<blocks, kCosetBlock, 0, stream>>>(p, out->steps - 1);
+  ++out->launches;
+  MG_CHECK_COSET(cudaGetLastError());
+  MG_CHECK_COSET(cudaStreamSynchronize(stream));
+  return MGBFS2_OK;
+}
+
 int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_count, cudaStream_t stream,
                CosetMemory* memory, CosetResult* out, DeviceBuffer* collect, uint64_t start_word) {
   const uint32_t count = static_cast<uint32_t>(jobs.size());
@@ -661,6 +986,18 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   const uint64_t warps = static_cast<uint64_t>(per_sm) * sm_count * kCosetWarps;
   uint32_t per_item = kMaxUnits;
   while (per_item > 1 && units / per_item < 6 * warps) per_item /= 2;
+  if (collect && !wide) {
+    // The small kernel where every unit gets a resident warp and 10! bounds the
+    // states (its layer sizes share a word with the barrier).
+    const size_t smem = static_cast<size_t>(kCosetWarps) * jobs[0].gens * 128 * sizeof(uint32_t);
+    int resident = 0;
+    if (jobs[0].n <= 10 && smem <= kSmallMaxShared &&
+        cudaFuncSetAttribute(coset_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmallMaxShared)) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, coset_small_kernel, kCosetBlock, smem) == cudaSuccess &&
+        units <= static_cast<uint64_t>(resident) * sm_count * kCosetWarps)
+      return coset_small(jobs[0], max_depth, static_cast<uint32_t>(units), smem, stream, memory, out, collect, start_word);
+    cudaGetLastError();
+  }
   std::vector<CosetInst> inst(count);
   std::vector<uint32_t> prefix(count + 1, 0);
   std::vector<uint8_t> perms;
@@ -799,16 +1136,7 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
     MG_CHECK_COSET(cudaMemcpyAsync(stamps.data(), p.stamps, 8ull * cols, cudaMemcpyDeviceToHost, stream));
     MG_CHECK_COSET(cudaStreamSynchronize(stream));
   }
-  out->layers.assign(count, {});
-  out->overflow.assign(count, 0);
-  for (uint32_t i = 0; i < count; ++i) {
-    const unsigned long long* row = counts.data() + static_cast<size_t>(i) * cols;
-    for (uint32_t d = 0; d < cols && row[d]; ++d) out->layers[i].push_back(row[d]);
-    out->overflow[i] = out->layers[i].size() > max_depth;
-  }
-  out->step_seconds.clear();
-  for (uint32_t d = 0; d + 1 < cols; ++d) out->step_seconds.push_back(static_cast<double>(stamps[d + 1] - stamps[d]) * 1e-9);
-  out->kernel_seconds = cols > 1 ? static_cast<double>(stamps[cols - 1] - stamps[0]) * 1e-9 : 0.0;
+  read_layers(counts, stamps, count, cols, max_depth, out);
   if (!collect || out->fatal || out->overflow[0]) return MGBFS2_OK;
   const CosetReport& r = *p.report;
   out->previous_small.assign(r.previous, r.previous + r.previous_count);
