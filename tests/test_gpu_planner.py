@@ -165,3 +165,71 @@ def test_learned_underprediction_grows_the_quotient_table():
         r = e.run()
     assert info["table_slot_bytes"] == 4 and info["table_slots"] == 4096
     assert r.complete and r.layer_sizes == golden("lrx_layers.json")["layers"]["9"]
+
+
+def _fp32_units(weights, bias, h):
+    """Which units a chain of fp32 fused multiply-adds in index order turns on
+    (a float64 product and sum, rounded once a term)."""
+    a = np.broadcast_to(bias, (len(h), len(bias))).astype(np.float32)
+    for k in range(h.shape[1]):
+        a = (weights[:, k].astype(np.float64) * h[:, k, None].astype(np.float64) + a).astype(np.float32)
+    return np.maximum(a, np.float32(0.0)), a > 0
+
+
+@pytest.mark.parametrize("inputs", [1, 16, 32])
+@pytest.mark.parametrize("rows", [1, 31, 32, 33, 9473])
+def test_loss_grad_tiles(inputs, rows):
+    """The tiled gradient at the edges of its tiles (32 rows, up to 32 inputs,
+    more tiles than blocks) against float64 with the units that fp32 turns on
+    (among 1.2 M pre-activations one can lie within rounding of zero); fp32 sums
+    of `rows` terms of order one stay within 2e-6 of their scale.  Added to what
+    grad and loss held."""
+    import torch
+    from multigpubfs_b200 import native
+    lib = native.require_device()
+    rng = np.random.default_rng(rows + inputs)
+    count = int(lib.mgbfs2_mlp_param_count(inputs))
+    params = rng.normal(0.0, 0.3, count).astype(np.float32)
+    x = rng.normal(size=(rows, inputs)).astype(np.float32)
+    t = rng.normal(size=(rows, 2)).astype(np.float32)
+    dev = [torch.tensor(a, device="cuda") for a in (params, x, t)]
+    grad, loss = torch.ones(count, device="cuda"), torch.ones(1, device="cuda")
+    rc = lib.mgbfs2_mlp_loss_grad(inputs, dev[0].data_ptr(), dev[1].data_ptr(), dev[2].data_ptr(), 1.0, 0.5, rows,
+                                  grad.data_ptr(), loss.data_ptr(), native.stream_handle())
+    assert rc == 0
+    w1, b1, w2, b2, w3, b3 = M.split(params, inputs)
+    h1, on1 = _fp32_units(w1, b1, x)
+    _, on2 = _fp32_units(w2, b2, h1)
+    y64, (x64, a1, _, a2, _) = M.forward(params.astype(np.float64), x, inputs)
+    h1, h2 = a1 * on1, a2 * on2
+    e = y64 - t
+    loss64 = float((np.array([1.0, 0.5]) * e * e).sum() / rows)
+    dy = 2.0 / rows * np.array([1.0, 0.5]) * e
+    d2 = (dy @ w3) * on2
+    d1 = (d2 @ w2) * on1
+    grad64 = np.concatenate([(d1.T @ x64).ravel(), d1.sum(0), (d2.T @ h1).ravel(), d2.sum(0), (dy.T @ h2).ravel(),
+                             dy.sum(0)])
+    got = grad.cpu().numpy().astype(np.float64) - 1.0
+    assert abs(float(loss.item()) - 1.0 - loss64) <= 2e-6 * (1.0 + abs(loss64))
+    assert np.abs(got - grad64).max() <= 2e-6 * (1.0 + np.abs(grad64).max())
+
+
+def test_loss_grad_leaves_out_products_with_zero():
+    """An infinite input on a row whose hidden units are off (relu 0) must not
+    turn their gradients into NaN."""
+    import torch
+    from multigpubfs_b200 import native
+    lib = native.require_device()
+    inputs, rows = 4, 40
+    count = int(lib.mgbfs2_mlp_param_count(inputs))
+    rng = np.random.default_rng(3)
+    params = rng.normal(0.0, 0.3, count).astype(np.float32)
+    params[:64 * inputs] = -np.abs(params[:64 * inputs])  # an input of +inf turns every first-layer unit off
+    x = rng.normal(size=(rows, inputs)).astype(np.float32)
+    x[7, 2] = np.inf
+    t = rng.normal(size=(rows, 2)).astype(np.float32)
+    dev = [torch.tensor(a, device="cuda") for a in (params, x, t)]
+    grad, loss = torch.zeros(count, device="cuda"), torch.zeros(1, device="cuda")
+    assert lib.mgbfs2_mlp_loss_grad(inputs, dev[0].data_ptr(), dev[1].data_ptr(), dev[2].data_ptr(), 1.0, 1.0, rows,
+                                    grad.data_ptr(), loss.data_ptr(), native.stream_handle()) == 0
+    assert bool(torch.isfinite(grad).all()) and bool(torch.isfinite(loss).all())
