@@ -67,6 +67,9 @@ struct RouteParams {
   // so each rank's buckets are contiguous (owner-major, block-minor).
   uint32_t owners, owner_blocks;
   MatrixAction mat;  // packed modular matrices (route_lehmer<kRadixDomain, 1>)
+  // count_lehmer: the parent positions that a generator's child has first and
+  // second, four bits each.
+  uint8_t heads[64];
 };
 
 struct AcceptParams {
@@ -92,8 +95,9 @@ struct AcceptParams {
 
 // Shard of a successor: its rank range for the Lehmer bitmap, or (N = 0) the
 // table region of its home slot for the hash.
+// `bucket` maps a prefix block to its bucket (bucket_table).
 template <int N, int K>
-__device__ __forceinline__ uint32_t route_shard(const RouteParams& p, uint64_t c);
+__device__ __forceinline__ uint32_t route_shard(const RouteParams& p, uint64_t c, const uint8_t* bucket);
 
 // Dynamic shared memory of route_lehmer (after the generator program).
 struct RouteSmem {
@@ -119,16 +123,22 @@ __device__ __forceinline__ uint32_t prefix_shard(uint64_t w) {
   return shard;
 }
 
+// Buckets of the prefix blocks, in shared memory: the owner and local block of
+// a block are two divisions by the number of ranks, too many for every child.
+__device__ __forceinline__ void bucket_table(const RouteParams& p, uint8_t* bucket) {
+  for (uint32_t s = threadIdx.x; s < kMaxShards; s += blockDim.x)
+    bucket[s] = static_cast<uint8_t>(p.owners > 1 ? (s % p.owners) * p.owner_blocks + s / p.owners : s);
+}
+
 template <int N, int K>
-__device__ __forceinline__ uint32_t route_shard(const RouteParams& p, uint64_t c) {
+__device__ __forceinline__ uint32_t route_shard(const RouteParams& p, uint64_t c, const uint8_t* bucket) {
   if constexpr (N == kRadixDomain) {
     const uint32_t top = p.mat.rows * p.mat.cols - 1;
     return static_cast<uint32_t>((c >> (p.mat.bits * top)) & ((1ull << p.mat.bits) - 1));
   } else if constexpr (N == 0) {
     return static_cast<uint32_t>((mix64(c & p.key_mask) & p.table_mask) >> p.region_shift);
   } else {
-    const uint32_t s = prefix_shard<N, K>(c);
-    return p.owners > 1 ? (s % p.owners) * p.owner_blocks + s / p.owners : s;
+    return bucket[prefix_shard<N, K>(c)];
   }
 }
 
@@ -140,6 +150,8 @@ __global__ void __launch_bounds__(kBlock, 3) route_lehmer(RouteParams p) {
   uint32_t* tbegin = reinterpret_cast<uint32_t*>(dyn_smem + sizeof(RouteSmem) + p.total_terms * sizeof(Term));
   for (uint32_t i = threadIdx.x; i < p.total_terms; i += blockDim.x) terms[i] = p.terms[i];
   for (uint32_t i = threadIdx.x; i <= 2 * p.gens; i += blockDim.x) tbegin[i] = p.term_begin[i];
+  __shared__ uint8_t bucket[kMaxShards];
+  if constexpr (N > 0) bucket_table(p, bucket);
   const uint32_t* inverse = tbegin + p.gens + 1;
   for (uint32_t i = threadIdx.x; i < kWarpsPerBlock * kMaxShards; i += blockDim.x) (&sm.hist[0][0])[i] = 0;
   __syncthreads();
@@ -193,7 +205,7 @@ __global__ void __launch_bounds__(kBlock, 3) route_lehmer(RouteParams p) {
             uint64_t c;
             if constexpr (N == kRadixDomain) c = apply_matrix(p.mat, par[k], terms, tb, te);
             else c = apply_terms(par[k], terms, tb, te);
-            const uint32_t s = route_shard<N, K>(p, c);
+            const uint32_t s = route_shard<N, K>(p, c, bucket);
             const uint32_t slot = live * kBlock + tid;
             sm.state[slot] = c | gtag;
             sm.tag[slot] = s | (atomicAdd(&sm.hist[warp][s], 1u) << 8);
@@ -294,18 +306,21 @@ __device__ __forceinline__ uint64_t lehmer_rank4_in_shard(uint64_t w, uint32_t s
 }
 
 // Counting pass for exactly sized buckets: the shard histogram of all
-// successors of the frontier (same generation and shard rule as route).
+// successors of the frontier (the shard rule of route).  The shard is the
+// child's first one or two symbols, which the parent holds at positions the
+// generator gives, so no child is made: two field reads in place of the
+// displacement terms.
 template <int N, int K>
 __global__ void __launch_bounds__(kBlock) count_lehmer(RouteParams p) {
+  static_assert(N > 0 && K <= 2, "permutations of distinct labels, shards of one or two symbols");
   extern __shared__ __align__(16) unsigned char dyn_smem[];
+  __shared__ uint8_t bucket[kMaxShards];
   uint32_t* hist = reinterpret_cast<uint32_t*>(dyn_smem);
-  Term* terms = reinterpret_cast<Term*>(dyn_smem + kMaxShards * sizeof(uint32_t));
-  uint32_t* tbegin = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(terms) + p.total_terms * sizeof(Term));
-  for (uint32_t i = threadIdx.x; i < p.total_terms; i += blockDim.x) terms[i] = p.terms[i];
-  for (uint32_t i = threadIdx.x; i <= 2 * p.gens; i += blockDim.x) tbegin[i] = p.term_begin[i];
+  uint32_t* inverse = hist + kMaxShards;
+  for (uint32_t i = threadIdx.x; i < p.gens; i += blockDim.x) inverse[i] = p.term_begin[p.gens + 1 + i];
   for (uint32_t s = threadIdx.x; s < p.shards; s += blockDim.x) hist[s] = 0;
+  bucket_table(p, bucket);
   __syncthreads();
-  const uint32_t* inverse = tbegin + p.gens + 1;
   for (unsigned long long i = blockIdx.x * static_cast<unsigned long long>(blockDim.x) + threadIdx.x; i < p.count;
        i += static_cast<unsigned long long>(gridDim.x) * blockDim.x) {
     const unsigned long long w = p.frontier[i];
@@ -313,10 +328,13 @@ __global__ void __launch_bounds__(kBlock) count_lehmer(RouteParams p) {
     const uint32_t skip = tag ? inverse[tag - 1] : 0xffffffffu;
     for (uint32_t g = 0; g < p.gens; ++g)
       if (g != skip) {
-        uint64_t c;
-        if constexpr (N == kRadixDomain) c = apply_matrix(p.mat, w, terms, tbegin[g], tbegin[g + 1]);
-        else c = apply_terms(w, terms, tbegin[g], tbegin[g + 1]);
-        atomicAdd(&hist[route_shard<N, K>(p, c)], 1u);
+        const uint32_t head = p.heads[g];
+        uint32_t s = static_cast<uint32_t>(w >> (4 * (head & 15u))) & 15u;
+        if constexpr (K == 2) {
+          const uint32_t second = static_cast<uint32_t>(w >> (4 * (head >> 4))) & 15u;
+          s = s * static_cast<uint32_t>(N - 1) + second - (second > s ? 1u : 0u);
+        }
+        atomicAdd(&hist[bucket[s]], 1u);
       }
   }
   __syncthreads();

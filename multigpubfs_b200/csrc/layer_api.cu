@@ -38,18 +38,34 @@ LayerLayout layer_layout(uint64_t entries) {
 
 // Single block: begin = exclusive scan of the counts, cap = counts (exact),
 // then the counts and the accept work counter restart at zero.
-__global__ void layout_shards(unsigned long long* meta, uint32_t shards) {
-  if (threadIdx.x == 0) {
-    unsigned long long run = 0;
-    for (uint32_t s = 0; s < shards; ++s) {
-      const unsigned long long c = meta[2 * kMaxShards + s];
-      meta[s] = run;
-      meta[kMaxShards + s] = c;
-      meta[2 * kMaxShards + s] = 0;
-      run += c;
-    }
-    meta[3 * kMaxShards] = 0;
+// Exclusive scan of kMaxShards counts by one block of that many threads; a
+// thread walking them alone took 19 us a layer, several times what a layer of
+// a small search takes.
+__device__ __forceinline__ unsigned long long scan_shards(unsigned long long c) {
+  __shared__ unsigned long long sums[kMaxShards / 32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  unsigned long long incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long up = __shfl_up_sync(kFullMask, incl, o);
+    if (lane >= static_cast<uint32_t>(o)) incl += up;
   }
+  if (lane == 31) sums[warp] = incl;
+  __syncthreads();
+  unsigned long long base = 0;
+  for (uint32_t w = 0; w < warp; ++w) base += sums[w];
+  return base + incl - c;
+}
+
+__global__ void __launch_bounds__(kMaxShards) layout_shards(unsigned long long* meta, uint32_t shards) {
+  const uint32_t s = threadIdx.x;
+  const unsigned long long c = s < shards ? meta[2 * kMaxShards + s] : 0ull, begin = scan_shards(c);
+  if (s < shards) {
+    meta[s] = begin;
+    meta[kMaxShards + s] = c;
+    meta[2 * kMaxShards + s] = 0;
+  }
+  if (s == 0) meta[3 * kMaxShards] = 0;
 }
 
 __global__ void publish_layer(const Control* control, unsigned long long* next_count, unsigned int* error) {
@@ -163,10 +179,20 @@ int prepare_layer_program(uint32_t degree, uint32_t generators, const uint32_t* 
   return MGBFS2_OK;
 }
 
+// The positions count_lehmer reads for every generator.
+void set_heads(uint32_t degree, uint32_t generators, const uint32_t* perms, RouteParams* rp) {
+  static_assert(sizeof(rp->heads) >= kLayerMaxGens, "one head a generator");
+  for (uint32_t g = 0; g < generators; ++g) {
+    const uint32_t* s = perms + static_cast<size_t>(g) * degree;
+    rp->heads[g] = static_cast<uint8_t>(s[0] | (s[1] << 4));
+  }
+}
+
 // Enqueues count -> layout -> route -> accept -> publish on `stream`, with the
 // generator program already in scratch at l.program and the control block and
 // shard metadata already zeroed.  Both layer entry points end here.
-int enqueue_layer(const LayerProgram& prog, uint32_t degree, uint32_t generators, const uint64_t* frontier,
+int enqueue_layer(const LayerProgram& prog, uint32_t degree, uint32_t generators,
+                  const uint32_t* permutations_host, const uint64_t* frontier,
                   uint64_t count, uint64_t* bitmap, uint64_t* next, uint64_t next_capacity, uint64_t* next_count,
                   uint32_t* error, unsigned char* scratch, const LayerLayout& l, int device, cudaStream_t stream) {
   TraceRange range("layer_api.expand");
@@ -195,10 +221,11 @@ int enqueue_layer(const LayerProgram& prog, uint32_t degree, uint32_t generators
   const LayerKernels& k = prog.kernels;
   cudaError_t e = cudaSuccess;
   if (count) {
-    const size_t count_smem = kMaxShards * sizeof(uint32_t) + prog.bytes();
+    set_heads(degree, generators, permutations_host, &rp);
+    const size_t count_smem = (kMaxShards + kLayerMaxGens) * sizeof(uint32_t);
     k.count<<<occupancy_grid(reinterpret_cast<const void*>(k.count), count_smem, device), kBlock, count_smem,
               stream>>>(rp);
-    layout_shards<<<1, 32, 0, stream>>>(meta, rp.shards);
+    layout_shards<<<1, kMaxShards, 0, stream>>>(meta, rp.shards);
     const size_t route_smem = sizeof(RouteSmem) + prog.bytes();
     if ((e = cudaFuncSetAttribute(reinterpret_cast<const void*>(k.route), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(route_smem))) != cudaSuccess)
@@ -249,7 +276,7 @@ int expand_layer_into(uint32_t degree, uint32_t generators, const uint32_t* perm
       (e = cudaMemcpyAsync(program + prog.terms.size() * sizeof(Term), prog.begin.data(),
                            prog.begin.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, stream)) != cudaSuccess)
     return cuda_status(e);
-  return enqueue_layer(prog, degree, generators, frontier, count, bitmap, next, next_capacity, next_count, error,
+  return enqueue_layer(prog, degree, generators, permutations_host, frontier, count, bitmap, next, next_capacity, next_count, error,
                        scratch, l, device, stream);
 }
 
@@ -298,22 +325,18 @@ __global__ void publish_route(const Control* control, const unsigned long long* 
 // (source rank order); source r's segment holds its local blocks j in order,
 // counts[r * blocks + j] words each.  Accept bucket j * world + r (block-major,
 // so the resident blocks claim in one local block at a time) gets its range.
-__global__ void layout_incoming(const unsigned long long* counts, uint32_t world, uint32_t blocks,
-                                unsigned long long* meta) {
-  if (threadIdx.x == 0) {
-    unsigned long long run = 0;
-    for (uint32_t r = 0; r < world; ++r) {
-      for (uint32_t j = 0; j < blocks; ++j) {
-        const uint32_t b = j * world + r;
-        const unsigned long long c = counts[static_cast<size_t>(r) * blocks + j];
-        meta[b] = run;
-        meta[kMaxShards + b] = c;
-        meta[2 * kMaxShards + b] = c;
-        run += c;
-      }
-    }
-    meta[3 * kMaxShards] = 0;
+__global__ void __launch_bounds__(kMaxShards) layout_incoming(const unsigned long long* counts, uint32_t world,
+                                                              uint32_t blocks, unsigned long long* meta) {
+  // world * blocks <= kMaxShards: thread t holds source t / blocks, block t % blocks.
+  const uint32_t t = threadIdx.x, r = t / blocks, j = t - r * blocks;
+  const unsigned long long c = r < world ? counts[t] : 0ull, begin = scan_shards(c);
+  if (r < world) {
+    const uint32_t b = j * world + r;
+    meta[b] = begin;
+    meta[kMaxShards + b] = c;
+    meta[2 * kMaxShards + b] = c;
   }
+  if (t == 0) meta[3 * kMaxShards] = 0;
 }
 
 // Parent-edge tags of the owner-partitioned path: a child carries the number
@@ -404,11 +427,12 @@ int shard_route(uint32_t degree, uint32_t generators, const uint32_t* permutatio
     rp.shard_cap = meta + kMaxShards;
     rp.shard_count = meta + 2 * kMaxShards;
     rp.control = control;
+    set_heads(degree, generators, permutations_host, &rp);
     const LayerKernels& k = prog.kernels;
-    const size_t count_smem = kMaxShards * sizeof(uint32_t) + prog.bytes();
+    const size_t count_smem = (kMaxShards + kLayerMaxGens) * sizeof(uint32_t);
     k.count<<<occupancy_grid(reinterpret_cast<const void*>(k.count), count_smem, device), kBlock, count_smem,
               stream>>>(rp);
-    layout_shards<<<1, 32, 0, stream>>>(meta, buckets);
+    layout_shards<<<1, kMaxShards, 0, stream>>>(meta, buckets);
     const size_t route_smem = sizeof(RouteSmem) + prog.bytes();
     if ((e = cudaFuncSetAttribute(reinterpret_cast<const void*>(k.route), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(route_smem))) != cudaSuccess)
@@ -440,7 +464,7 @@ int shard_accept(uint32_t degree, uint32_t world, uint32_t owner, const uint64_t
   if (int rc = stage_program(LayerProgram{}, scratch, l, stream)) return rc;
   Control* control = reinterpret_cast<Control*>(scratch + l.control);
   unsigned long long* meta = reinterpret_cast<unsigned long long*>(scratch + l.meta);
-  layout_incoming<<<1, 32, 0, stream>>>(reinterpret_cast<const unsigned long long*>(incoming_counts), world,
+  layout_incoming<<<1, kMaxShards, 0, stream>>>(reinterpret_cast<const unsigned long long*>(incoming_counts), world,
                                         g.blocks_per_owner, meta);
   AcceptParams ap{};
   ap.buckets = reinterpret_cast<const unsigned long long*>(incoming);
@@ -557,7 +581,7 @@ int expand_layer_static(uint32_t degree, uint32_t generators, const uint32_t* pe
                                                reinterpret_cast<uint32_t*>(program + prog.terms.size()),
                                                reinterpret_cast<Control*>(scratch + l.control),
                                                reinterpret_cast<unsigned long long*>(scratch + l.meta));
-  return enqueue_layer(prog, degree, generators, frontier, count, bitmap, next, next_capacity, next_count, error,
+  return enqueue_layer(prog, degree, generators, permutations_host, frontier, count, bitmap, next, next_capacity, next_count, error,
                        scratch, l, device, stream);
 }
 
