@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #define MG_CHECK_COSET(expr)                       \
   do {                                             \
@@ -17,6 +18,7 @@ namespace {
 constexpr uint32_t kSlots = 7, kSlotPerms = 5040;
 constexpr uint32_t kCosetBlock = 256, kCosetWarps = kCosetBlock / 32;
 constexpr uint32_t kMaxUnits = 8;  // units (128 nodes) of a work item
+constexpr uint32_t kWideUnits = 4, kWideRows = 36;  // 64-bit words: units of an item, rows of a chunk
 constexpr size_t kSmallMaxShared = 160 << 10;  // parent words of a block of the small kernel
 
 struct CosetInst {
@@ -47,6 +49,7 @@ struct CosetParams {
   const uint32_t* item_prefix;  // count + 1: exclusive prefix of the jobs' work items
   const uint8_t* perms;
   uint32_t count, units;        // jobs; units per item (a power of two)
+  uint32_t chunk, spare;        // 64-bit words: items of a block's chunk
   uint32_t stride, max_steps;   // layer-table columns; last step that may run
   unsigned long long* counts;   // count x stride layer sizes
   uint32_t* active;             // stride: layer d of any job is not empty
@@ -307,6 +310,7 @@ __global__ void __launch_bounds__(kCosetBlock) coset_setup(CosetParams p) {
     uint32_t code, flips;
     const uint32_t parent = row_image(in.m, row, p.perms + in.perm_off + 16 * g, &code, &flips);
     p.used[code] = 1;
+    if (flips) p.used[0] = 1;  // read for rows that flip outer labels only
     p.desc[t] = parent | (static_cast<unsigned long long>(code) << 32) | (static_cast<unsigned long long>(flips) << 48);
   }
   for (unsigned long long i = thread; i < p.count; i += step) {
@@ -338,9 +342,9 @@ __device__ __forceinline__ uint32_t table_entry(uint32_t node, uint32_t flips) {
 // The table rows of the slot permutations that some row needs: the image of
 // every node and its inner flips.  One warp takes a permutation.
 template <typename W>
-__device__ void coset_table(const CosetParams& p) {
+__device__ void coset_table(const CosetParams& p, uint32_t per_block) {
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warps = gridDim.x * kCosetWarps, warp = blockIdx.x * kCosetWarps + (threadIdx.x >> 5);
+  const uint32_t warps = gridDim.x * per_block, warp = blockIdx.x * per_block + (threadIdx.x >> 5);
   for (uint32_t base = 0; base * warps + warp < kSlotPerms; base += 32) {
     const uint32_t mine = (base + lane) * warps + warp;
     uint32_t found = __ballot_sync(kFullMask, mine < kSlotPerms && __ldcg(p.used + mine));
@@ -386,6 +390,16 @@ __device__ __forceinline__ unsigned long long flip_outer(unsigned long long w, u
   if (q & 4u) lo = swap_bits(lo, 0x0f0f0f0fu, 4), hi = swap_bits(hi, 0x0f0f0f0fu, 4);
   return (static_cast<unsigned long long>(hi) << 32) | lo;
 }
+// Four words by one branch a flip (the flips are the same in all lanes).
+template <typename W>
+__device__ __forceinline__ void flip_words(W (&w)[4], uint32_t q) {
+#pragma unroll
+  for (uint32_t bit = 1; bit <= (sizeof(W) == 8 ? 4u : 2u); bit *= 2)
+    if (q & bit) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) w[k] = flip_outer(w[k], bit);
+    }
+}
 __device__ __forceinline__ uint32_t popcount(uint32_t w) { return __popc(w); }
 __device__ __forceinline__ uint32_t popcount(unsigned long long w) { return __popcll(w); }
 
@@ -398,8 +412,8 @@ __device__ __forceinline__ uint32_t lowest_bit(W b) {
 // d as packed words, in any order, and block 0 writes the report.
 template <typename W>
 __device__ void coset_finish(const CosetParams& p, const CosetInst& in, uint32_t d, bool exhausted) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warps = gridDim.x * kCosetWarps, warp = blockIdx.x * kCosetWarps + (threadIdx.x >> 5);
+  const uint32_t lane = threadIdx.x & 31u, per_block = blockDim.x / 32;
+  const uint32_t warps = gridDim.x * per_block, warp = blockIdx.x * per_block + (threadIdx.x >> 5);
   constexpr bool kWide = sizeof(W) == 8;
   CosetReport* r = p.report;
   const unsigned long long keep = (1ull << (4 * p.n)) - 1ull;  // embedded: positions from n up are not written
@@ -452,18 +466,27 @@ __device__ void coset_finish(const CosetParams& p, const CosetInst& in, uint32_t
   }
 }
 
+// Threads of a block: with 64-bit words a whole multiprocessor's.
+template <typename W>
+constexpr uint32_t coset_threads() {
+  return sizeof(W) == 8 ? 1024 : kCosetBlock;
+}
+
 // A whole search per launch: step d pulls layer d + 1 of every job, one grid
 // barrier ends it.  A work item is up to `units` units of one job; its warp
 // first looks, one lane per (unit, generator), which parent rows hold anything,
 // and skips units with none (early and last layers touch few rows).
 template <typename W>
-__global__ void __launch_bounds__(kCosetBlock, 4) coset_wave_kernel(CosetParams p) {
+__global__ void __launch_bounds__(coset_threads<W>(), 1024 / coset_threads<W>()) coset_wave_kernel(CosetParams p) {
+  constexpr uint32_t kWarps = coset_threads<W>() / 32;
+  __shared__ uint32_t tickets[2];
   const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warps = gridDim.x * kCosetWarps, warp = blockIdx.x * kCosetWarps + (threadIdx.x >> 5);
+  const uint32_t warps = gridDim.x * kWarps, warp = blockIdx.x * kWarps + (threadIdx.x >> 5);
   const uint32_t items = p.item_prefix[p.count];
   const uint32_t unit_mask = p.units - 1u;
   uint32_t epoch = 0;
-  coset_table<W>(p);
+  if (threadIdx.x == 0) tickets[0] = 0;
+  coset_table<W>(p, kWarps);
   if (!arrival_barrier(&p.ctl->arrived, &p.ctl->error, &epoch)) return;
   CosetInst in = p.inst[0];
   for (uint32_t d = 0;; ++d) {
@@ -493,11 +516,26 @@ __global__ void __launch_bounds__(kCosetBlock, 4) coset_wave_kernel(CosetParams 
     // three quarters of the items fixed).  A layer with fewer states than items
     // skips nearly all of them, which the counter would only slow (S13: 39 ->
     // 67 us for an empty one): those go round the warps.
-    const bool counter = p.count > 1 || __ldcg(p.counts + d) >= items;
-    uint32_t item = warp;
+    // 64-bit words: a block is all of a multiprocessor and its warps share a
+    // chunk of neighbouring rows, whose parents largely coincide: what one warp
+    // has read the others find in L1.  L2 gives the multiprocessors 5 to 6 TB/s
+    // (bulk copies of whole rows reach no more), which is what such a layer waits for.
+    constexpr bool kChunks = sizeof(W) == 8;
+    const bool counter = !kChunks && (p.count > 1 || __ldcg(p.counts + d) >= items);
+    if (kChunks && threadIdx.x == 0) tickets[(d + 1) & 1u] = 0;
+    const auto take = [&]() {
+      uint32_t t = 0;
+      if (lane == 0) t = atomicAdd(&tickets[d & 1u], 1u);
+      t = __shfl_sync(kFullMask, t, 0);
+      const uint32_t c = t / p.chunk;
+      return (blockIdx.x + c * gridDim.x) * p.chunk + t - c * p.chunk;
+    };
+    uint32_t item = kChunks ? take() : warp;
     for (uint32_t coming; item < items; item = coming) {
       coming = item + warps;
-      if (counter) {
+      if (kChunks) {
+        coming = take();
+      } else if (counter) {
         if (lane == 0) coming = warps + atomicAdd(p.next_item + d, 1u);
         coming = __shfl_sync(kFullMask, coming, 0);
       }
@@ -542,41 +580,142 @@ __global__ void __launch_bounds__(kCosetBlock, 4) coset_wave_kernel(CosetParams 
           from_row = static_cast<uint32_t>(e);
           how = static_cast<uint32_t>(e >> 32);
         }
-        // Generators that keep the free positions' order read the parent row
-        // as it lies; the others through their table row, two at a time, so
-        // that eight gathers are in flight.
-        const uint32_t moved = __ballot_sync(kFullMask, (how & 0xffffu) != 0) & mask, kept = mask & ~moved;
+        // Generators that keep the free positions' order and every outer pair's
+        // read the parent row as it lies, the others through their table row, two
+        // at a time: eight loads in flight and one three-way OR for both.  The
+        // integer pipe, at half the issue rate, bounds a full layer, and a flip
+        // that is only predicated off still takes its slots: with one loop for
+        // all generators 25 instructions a word and generator and the pipe at
+        // 84 % on S13, adjacent transpositions (52.0 ms, 24.4 ms in these loops).
+        // With 64-bit words those without outer flips go by themselves (31.9 ms
+        // otherwise) and an odd one out is done twice (26.3 ms with its own tail,
+        // which spills); with 32-bit words the reverse (eight S12 instances: 11.0
+        // ms; 12.4 ms the other way).
+        const uint32_t plain = __ballot_sync(kFullMask, how == 0) & mask;
         W acc[4] = {0, 0, 0, 0};
-        for (uint32_t left = kept; left; left &= left - 1u) {
-          const int g = __ffs(static_cast<int>(left)) - 1;
-          const uint32_t q = __shfl_sync(kFullMask, how, g) >> 16;
-          const W* from = cur + (in.row_off + __shfl_sync(kFullMask, from_row, g)) * kCosetStride + x0;
-          W w[4];
+        if constexpr (sizeof(W) == 8) {
+          const uint32_t flipped = __ballot_sync(kFullMask, (how >> 16) != 0) & mask;
+          for (uint32_t left = plain; left;) {
+            const int g = __ffs(static_cast<int>(left)) - 1;
+            left &= left - 1u;
+            const W* from_g = cur + (in.row_off + __shfl_sync(kFullMask, from_row, g)) * kCosetStride + x0;
+            const int h = left ? __ffs(static_cast<int>(left)) - 1 : g;
+            left &= left - 1u;
+            const W* from_h = cur + (in.row_off + __shfl_sync(kFullMask, from_row, h)) * kCosetStride + x0;
+            W w_g[4], w_h[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) w[k] = from[32 * k];
+            for (int k = 0; k < 4; ++k) w_g[k] = from_g[32 * k], w_h[k] = from_h[32 * k];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) acc[k] |= flip_outer(w[k], q);
-        }
-        for (uint32_t left = moved; left;) {
-          const int g = __ffs(static_cast<int>(left)) - 1;
-          left &= left - 1u;
-          const int h = left ? __ffs(static_cast<int>(left)) - 1 : g;  // an odd one out is taken twice
-          left &= left - 1u;
-          const uint32_t how_g = __shfl_sync(kFullMask, how, g), how_h = __shfl_sync(kFullMask, how, h);
-          const W* from_g = cur + (in.row_off + __shfl_sync(kFullMask, from_row, g)) * kCosetStride;
-          const W* from_h = cur + (in.row_off + __shfl_sync(kFullMask, from_row, h)) * kCosetStride;
-          const uint32_t* table_g = p.table + (how_g & 0xffffu) * kCosetStride + x0;
-          const uint32_t* table_h = p.table + (how_h & 0xffffu) * kCosetStride + x0;
-          uint32_t to_g[4], to_h[4];
-          W w_g[4], w_h[4];
+            for (int k = 0; k < 4; ++k) acc[k] |= w_g[k] | w_h[k];
+          }
+          for (uint32_t left = mask & ~plain & ~flipped; left;) {
+            const int g = __ffs(static_cast<int>(left)) - 1;
+            left &= left - 1u;
+            const uint32_t how_g = __shfl_sync(kFullMask, how, g);
+            const W* from_g = cur + (in.row_off + __shfl_sync(kFullMask, from_row, g)) * kCosetStride;
+            const uint32_t* table_g = p.table + (how_g & 0xffffu) * kCosetStride + x0;
+            uint32_t to_g[4];
+            W w_g[4];
+            const int h = left ? __ffs(static_cast<int>(left)) - 1 : g;
+            left &= left - 1u;
+            const uint32_t how_h = __shfl_sync(kFullMask, how, h);
+            const W* from_h = cur + (in.row_off + __shfl_sync(kFullMask, from_row, h)) * kCosetStride;
+            const uint32_t* table_h = p.table + (how_h & 0xffffu) * kCosetStride + x0;
+            uint32_t to_h[4];
+            W w_h[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) to_g[k] = table_g[32 * k], to_h[k] = table_h[32 * k];
+            for (int k = 0; k < 4; ++k) to_g[k] = table_g[32 * k], to_h[k] = table_h[32 * k];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) w_g[k] = from_g[to_g[k] >> 21], w_h[k] = from_h[to_h[k] >> 21];
+            for (int k = 0; k < 4; ++k) w_g[k] = from_g[to_g[k] >> 21], w_h[k] = from_h[to_h[k] >> 21];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) acc[k] |= flip_outer(flip_inner(w_g[k], to_g[k]), how_g >> 16);
+            for (int k = 0; k < 4; ++k) w_g[k] = flip_inner(w_g[k], to_g[k]), w_h[k] = flip_inner(w_h[k], to_h[k]);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) acc[k] |= flip_outer(flip_inner(w_h[k], to_h[k]), how_h >> 16);
+            for (int k = 0; k < 4; ++k) acc[k] |= w_g[k] | w_h[k];
+          }
+          // (The identity's table row for those that only flip.)
+          for (uint32_t left = flipped; left;) {
+            const int g = __ffs(static_cast<int>(left)) - 1;
+            left &= left - 1u;
+            const uint32_t how_g = __shfl_sync(kFullMask, how, g);
+            const W* from_g = cur + (in.row_off + __shfl_sync(kFullMask, from_row, g)) * kCosetStride;
+            const uint32_t* table_g = p.table + (how_g & 0xffffu) * kCosetStride + x0;
+            uint32_t to_g[4];
+            W w_g[4];
+            const int h = left ? __ffs(static_cast<int>(left)) - 1 : g;
+            left &= left - 1u;
+            const uint32_t how_h = __shfl_sync(kFullMask, how, h);
+            const W* from_h = cur + (in.row_off + __shfl_sync(kFullMask, from_row, h)) * kCosetStride;
+            const uint32_t* table_h = p.table + (how_h & 0xffffu) * kCosetStride + x0;
+            uint32_t to_h[4];
+            W w_h[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) to_g[k] = table_g[32 * k], to_h[k] = table_h[32 * k];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w_g[k] = from_g[to_g[k] >> 21], w_h[k] = from_h[to_h[k] >> 21];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w_g[k] = flip_inner(w_g[k], to_g[k]), w_h[k] = flip_inner(w_h[k], to_h[k]);
+            flip_words(w_g, how_g >> 16);
+            flip_words(w_h, how_h >> 16);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[k] |= w_g[k] | w_h[k];
+          }
+        } else {
+          for (uint32_t left = plain; left;) {
+            const int g = __ffs(static_cast<int>(left)) - 1;
+            left &= left - 1u;
+            const W* from_g = cur + (in.row_off + __shfl_sync(kFullMask, from_row, g)) * kCosetStride + x0;
+            if (!left) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) acc[k] |= from_g[32 * k];
+              break;
+            }
+            const int h = __ffs(static_cast<int>(left)) - 1;
+            left &= left - 1u;
+            const W* from_h = cur + (in.row_off + __shfl_sync(kFullMask, from_row, h)) * kCosetStride + x0;
+            W w_g[4], w_h[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w_g[k] = from_g[32 * k], w_h[k] = from_h[32 * k];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[k] |= w_g[k] | w_h[k];
+          }
+          for (uint32_t left = mask & ~plain; left;) {
+            const int g = __ffs(static_cast<int>(left)) - 1;
+            left &= left - 1u;
+            const uint32_t how_g = __shfl_sync(kFullMask, how, g);
+            const W* from_g = cur + (in.row_off + __shfl_sync(kFullMask, from_row, g)) * kCosetStride;
+            const uint32_t* table_g = p.table + (how_g & 0xffffu) * kCosetStride + x0;
+            uint32_t to_g[4];
+            W w_g[4];
+            if (!left) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) to_g[k] = table_g[32 * k];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) w_g[k] = from_g[to_g[k] >> 21];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) w_g[k] = flip_inner(w_g[k], to_g[k]);
+              flip_words(w_g, how_g >> 16);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) acc[k] |= w_g[k];
+              break;
+            }
+            const int h = __ffs(static_cast<int>(left)) - 1;
+            left &= left - 1u;
+            const uint32_t how_h = __shfl_sync(kFullMask, how, h);
+            const W* from_h = cur + (in.row_off + __shfl_sync(kFullMask, from_row, h)) * kCosetStride;
+            const uint32_t* table_h = p.table + (how_h & 0xffffu) * kCosetStride + x0;
+            uint32_t to_h[4];
+            W w_h[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) to_g[k] = table_g[32 * k], to_h[k] = table_h[32 * k];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w_g[k] = from_g[to_g[k] >> 21], w_h[k] = from_h[to_h[k] >> 21];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w_g[k] = flip_inner(w_g[k], to_g[k]), w_h[k] = flip_inner(w_h[k], to_h[k]);
+            flip_words(w_g, how_g >> 16);
+            flip_words(w_h, how_h >> 16);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[k] |= w_g[k] | w_h[k];
+          }
         }
         const unsigned long long own = (in.row_off + row) * kCosetStride + x0;
         W old[4] = {0, 0, 0, 0};
@@ -974,8 +1113,9 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   const size_t word = wide ? 8 : 4;
   const void* kernel = wide ? reinterpret_cast<const void*>(coset_wave_kernel<unsigned long long>)
                             : reinterpret_cast<const void*>(coset_wave_kernel<uint32_t>);
+  const uint32_t threads = wide ? coset_threads<unsigned long long>() : coset_threads<uint32_t>();
   int per_sm = 0;
-  MG_CHECK_COSET(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kCosetBlock, 0));
+  MG_CHECK_COSET(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, static_cast<int>(threads), 0));
   if (per_sm < 1) return MGBFS2_UNSUPPORTED;
   // Units per item: eight, fewer while that leaves warps without an item.
   uint64_t units = 0;
@@ -983,9 +1123,10 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
     if (!coset_supported(j.n, j.gens) || coset_wide(j.n) != wide || !j.perms) return MGBFS2_INVALID_ARGUMENT;
     units += static_cast<uint64_t>(rows_of(embedded(j.n))) * kCosetParts;
   }
-  const uint64_t warps = static_cast<uint64_t>(per_sm) * sm_count * kCosetWarps;
+  const uint64_t warps = static_cast<uint64_t>(per_sm) * sm_count * (threads / 32);
   uint32_t per_item = kMaxUnits;
   while (per_item > 1 && units / per_item < 6 * warps) per_item /= 2;
+  if (wide) per_item = kWideUnits;
   if (collect && !wide) {
     // The small kernel where every unit gets a resident warp and 10! bounds the
     // states (its layer sizes share a word with the barrier).
@@ -1070,6 +1211,7 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   p.perms = reinterpret_cast<const uint8_t*>(base + o_perms);
   p.count = count;
   p.units = per_item;
+  p.chunk = kWideRows * kCosetParts / kWideUnits;
   p.stride = stride;
   p.max_steps = max_depth - 1;
   p.counts = reinterpret_cast<unsigned long long*>(base + o_counts);
@@ -1100,7 +1242,8 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   if (e == cudaSuccess) e = cudaMemsetAsync(base + upload, 0, cleared - upload, stream);
   for (int k = 0; k < 3 && own && e == cudaSuccess; ++k)
     if (word_bytes[k]) e = cudaMemsetAsync(words[k], 0, word_bytes[k], stream);
-  const uint64_t blocks = std::min<uint64_t>((prefix[count] + kCosetWarps - 1) / kCosetWarps,
+  const uint32_t per_block = wide ? p.chunk : kCosetWarps;
+  const uint64_t blocks = std::min<uint64_t>((prefix[count] + per_block - 1) / per_block,
                                              static_cast<uint64_t>(per_sm) * sm_count);
   if (e == cudaSuccess) {
     const uint32_t setup = static_cast<uint32_t>(
@@ -1111,7 +1254,7 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   }
   if (e == cudaSuccess) {
     void* args[] = {&p};
-    e = cudaLaunchCooperativeKernel(kernel, dim3(static_cast<uint32_t>(blocks)), dim3(kCosetBlock), args, 0, stream);
+    e = cudaLaunchCooperativeKernel(kernel, dim3(static_cast<uint32_t>(blocks)), dim3(threads), args, 0, stream);
   }
   CosetCtl ctl{};
   if (e == cudaSuccess && !collect) e = cudaMemcpyAsync(&ctl, p.ctl, sizeof(ctl), cudaMemcpyDeviceToHost, stream);
