@@ -61,7 +61,14 @@ enum { MGBFS2_VISITED_AUTO = 0, MGBFS2_VISITED_BITMAP = 1, MGBFS2_VISITED_HASH =
 /* SORT: per-tile radix sort + unique of the children before the visited test.
  * BUCKET: route successors to rank-range shard buckets, then claim per shard.
  * GROUPED: claim first, route only the winners into a frontier grouped by its
- * first N-10 symbols (Lehmer bitmaps of degree 11..14). */
+ * first N-10 symbols (Lehmer bitmaps of degree 11..14).
+ * AUTO names one of these for layers over frontier lists (runs with limits, a
+ * callback or a resumed checkpoint, plans that set a capacity, a shape or the
+ * host loop) and runs a whole search without frontier lists where it can:
+ * distinct labels up to degree 14 and 32 generators in coset-word layers,
+ * inverse-closed invertible 2x2 matrices over primes 17..257 in unipotent-ring layers, up to
+ * six repeated labels in half-rank layers (csrc/coset.h, ring.h, half.h).  The
+ * results are the same. */
 enum { MGBFS2_DEDUP_AUTO = 0, MGBFS2_DEDUP_ATOMIC = 1, MGBFS2_DEDUP_WARP = 2, MGBFS2_DEDUP_SORT = 3,
        MGBFS2_DEDUP_BUCKET = 4, MGBFS2_DEDUP_GROUPED = 5 };
 enum { MGBFS2_PLANNER_PLAIN = 0, MGBFS2_PLANNER_LEARNED = 1 };
@@ -459,8 +466,11 @@ typedef struct {
 MGBFS2_API int mgbfs2_batch_create(const mgbfs2_graph_desc* graphs, uint32_t count, int device, mgbfs2_batch** out,
                                    char* error, size_t error_capacity);
 
-/* Runs every instance to completion in waves that fit the memory budget.  By
- * default a wave is ONE persistent cooperative launch that expands every active
+/* Runs every instance to completion in waves that fit the memory budget.  With
+ * default options a wave of instances up to degree 14 is ONE persistent
+ * cooperative launch in coset-word layers (csrc/coset.h).  Otherwise (a
+ * degree-15 instance, predicted capacities, explicit shapes) it is ONE
+ * persistent cooperative launch that expands every active
  * instance's layer, finalizes it behind a bounded grid barrier and repeats
  * until the device finds no active instance (options->host_loop selects the
  * CUDA-graph WHILE form or a host-driven loop instead).  With predicted

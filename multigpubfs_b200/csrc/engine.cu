@@ -1328,16 +1328,21 @@ int Graph::make_plan(const mgbfs2_plan_request* req, mgbfs2_plan_info* out) {
              !r.parents_per_thread && !r.route_chunk && !r.bucket_min_work && !r.bucket_margin &&
              (!orbit_bound || orbit_bound >= rank_total) && coset_supported(elements, gens) &&
              coset_job_bytes(job, kWholeDepth) + coset_fixed_bytes(kWholeDepth) <= budget / 2;
-  // Likewise 2x2 matrices over a prime field in scalar-ring layers (ring.h),
-  // from the layer on where they overtake the list layers.
+  // Likewise invertible 2x2 matrices over a prime field in unipotent-ring
+  // layers (ring.h), from the layer on where they overtake the list layers.  A
+  // singular start reaches fewer than p^2 states.
   bool ring_field = packed_matrix && rows == 2 && cols == 2 && moduli[0] >= kRingMinPrime &&
-                    moduli[0] <= kRingMaxPrime && start_word;
+                    moduli[0] <= kRingMaxPrime;
+  if (ring_field) {
+    const auto entry = [&](uint32_t i) { return (start_word >> (i * bits)) & ((1ull << bits) - 1); };
+    ring_field = entry(0) * entry(3) % moduli[0] != entry(1) * entry(2) % moduli[0];
+  }
   for (uint32_t q = 2; ring_field && q * q <= moduli[0]; ++q) ring_field = moduli[0] % q != 0;
   ring_ok = ring_field && visited == MGBFS2_VISITED_BITMAP && r.dedup == MGBFS2_DEDUP_AUTO && inverse_closed &&
             !host_loop_only && !r.capacity && !r.shards && !r.blocks_per_sm && !r.parents_per_thread &&
             !r.route_chunk && !r.bucket_min_work && !r.bucket_margin && gens <= kRingMaxGens &&
             (!orbit_bound || orbit_bound >= rank_total) &&
-            ring_bytes(moduli[0], kWholeDepth) + bitmap_bytes <= budget / 2;
+            ring_bytes(moduli[0], gens, kWholeDepth) + bitmap_bytes <= budget / 2;
   // Permutations with repeated labels in half-rank layers (half.h): packed ones
   // in place of the fused multinomial bitmap layers, starts of more than 16
   // positions in place of the wide hash where the bitmap is small and not much

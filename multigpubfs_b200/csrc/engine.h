@@ -198,7 +198,7 @@ struct Graph {
 
   // Searches without frontier lists (whole_search.cu): the default plan of a
   // Lehmer bitmap in coset-word layers (coset.h), of 2x2 matrices over a prime
-  // field in scalar-ring layers (ring.h), of repeated labels in half-rank
+  // field in unipotent-ring layers (ring.h), of repeated labels in half-rank
   // layers (half.h; half_rows: their samples of wide states).  no_bitmap: `bitmap` does not hold
   // the last run's visited states (a checkpoint runs the list layers first).
   CosetMemory* coset = nullptr;

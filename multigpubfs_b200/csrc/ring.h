@@ -1,19 +1,22 @@
-// Scalar-ring layers: exact BFS of 2x2 matrices over a prime field with the
-// frontier as one bit ring per matrix up to a scalar.
+// Unipotent-ring layers: exact BFS of invertible 2x2 matrices over a prime field
+// with the frontier as one bit ring per first column and determinant.
 //
-// Scalars commute with every generator, so the p - 1 nonzero multiples of a
-// matrix share a ring of p - 1 bits (bit t = g^t times the node's matrix, g a
-// primitive root) and a generator maps a ring onto a ring, rotated by the
-// discrete logarithm of the scalar that makes the product canonical: one
-// 2x2 product, one 32-byte load and one rotation carry p - 1 edges.  The list
-// layers (packed_kernels.cuh, bucket_kernels.cuh) do a product, a rank and an
-// atomic for each edge.
+// Generators multiply from the left, so the p matrices that differ by a column
+// operation (the second column plus t times the first) share a ring of p bits
+// and a generator maps a ring onto a ring, rotated: one table entry, one load of
+// the ring and one rotation carry p edges.  The list layers (packed_kernels.cuh,
+// bucket_kernels.cuh) do a product, a rank and an atomic for each edge.
 //
-// Node: a nonzero matrix (a b; c d) whose first nonzero entry in the order a,
-// c, b, d is 1.  Index, with a = 1: (c p + b) p + d, then the p^2 nodes with a
-// = 0, c = 1, then a = c = 0, b = 1, then d = 1.  The first column decides the
-// block of p^2 nodes, and generators act on columns: a block's parents come
-// from one block per generator, read whole.
+// Node: the determinant, then the first column (a, c) as a p + c - 1.  Bit t is
+// the second column w + t (a, c), with w = (0, det / a), or (-det / c, 0) where a
+// is 0.  A generator m leads from (v, det) to (m v, det m det); its shift is
+// det times a number of v and m alone, so one table of moves serves all
+// determinants.
+//
+// Nodes are kept by determinant because a layer holds few of them where the
+// generators' determinants generate the group slowly (a diagonal generator, or
+// none but 1): a pass visits the determinants that layer d leads to, 8 % of the
+// work at GL(2,211).
 //
 // A layer is pulled as in coset.h: inverse-closed sets only, two buffers, layer
 // d + 1 in the place of layer d - 1.
@@ -28,7 +31,7 @@
 namespace mgbfs2 {
 
 constexpr uint32_t kRingMaxGens = 32;
-constexpr uint32_t kRingMinPrime = 17, kRingMaxPrime = 257;  // rings of 16 to 256 bits
+constexpr uint32_t kRingMinPrime = 17, kRingMaxPrime = 257;  // rings of 17 to 257 bits
 constexpr uint32_t kRingSmall = 1000;  // layers of fewer states are kept for samples
 
 struct RingMemory {
@@ -61,7 +64,7 @@ struct RingResult {
 };
 
 uint64_t ring_nodes(uint32_t p);
-uint64_t ring_bytes(uint32_t p, uint32_t max_layers);
+uint64_t ring_bytes(uint32_t p, uint32_t gens, uint32_t max_layers);
 
 // Goes on from a frontier list (`front`, `count` packed words of `bits`-bit
 // entries) and the list of the layer before it (`before`, `before_count`, may
