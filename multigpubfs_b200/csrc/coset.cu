@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <numeric>
 #include <type_traits>
 
 #define MG_CHECK_COSET(expr)                       \
@@ -21,10 +22,13 @@ constexpr uint32_t kMaxUnits = 8;  // units (128 nodes) of a work item
 constexpr uint32_t kWideUnits = 4, kWideRows = 36;  // 64-bit words: units of an item, rows of a chunk
 constexpr size_t kSmallMaxShared = 160 << 10;  // parent words of a block of the small kernel
 
+constexpr uint32_t kNoWalk = 0xffffffffu;
+
 struct CosetInst {
   uint32_t m, gens, rows, inverse_closed;
   uint32_t same_layer;  // some generator is an even permutation: a layer may have edges inside it
   uint32_t perm_off;    // first byte of gens x 16 position images
+  uint32_t walk;        // 64-bit words: the generator whose orbits order the rows, kNoWalk without one
   unsigned long long row_off, desc_off;  // first row in the buffers and flags; first descriptor
 };
 
@@ -56,6 +60,8 @@ struct CosetParams {
   uint32_t* next_item;          // stride: work items of step d taken so far, past the first of every warp
   unsigned long long* stamps;   // stride: globaltimer at the start of step d
   uint8_t* used;                // slot permutations that some row needs
+  uint32_t* order;              // 64-bit words: every job's rows in the order they are visited
+  uint32_t* order_sums;         // rows of each setup block's orbits
   uint32_t* table;              // slot permutation x node -> image and flips (table_entry)
   unsigned long long* desc;     // row x generator -> parent row | slot permutation << 32 | outer flips << 48
   unsigned long long* flags[2]; // per row: byte p = part p of the buffer's row is not zero
@@ -328,6 +334,84 @@ __global__ void __launch_bounds__(kCosetBlock) coset_setup(CosetParams p) {
   if (thread == 0) p.active[0] = 1;
 }
 
+// The order in which a layer with 64-bit words visits its rows: orbit after
+// orbit of the job's generator of the greatest order, by their least row, so
+// that the rows it leads to and from are the neighbours in a chunk and are read
+// from L2 once.  S13 LRX (the shift's 13 rows an orbit): DRAM traffic 131 -> 86
+// GB, L2 sectors 7.3 -> 5.3 G, 28.3 -> 24.7 ms a call.  Without a generator
+// of order 3 or more the rank's order stays: orbits of two rows gain nothing
+// (adjacent transpositions: 25.9 ms either way).  Thread t of block b stands for row 1024 b +
+// t; the least row of an orbit places all of it, behind the orbits of smaller rows.
+constexpr uint32_t kOrderBlock = 1024;
+
+// Length of the orbit if the row is its least, else 0.
+__device__ __forceinline__ uint32_t orbit_of_least(const CosetParams& p, const CosetInst& in, uint32_t row) {
+  if (in.walk == kNoWalk) return 1;
+  uint32_t length = 0, at = row;
+  do {
+    at = static_cast<uint32_t>(p.desc[in.desc_off + static_cast<unsigned long long>(at) * in.gens + in.walk]);
+    ++length;
+    if (at < row) return 0;
+  } while (at != row);
+  return length;
+}
+
+__device__ __forceinline__ bool job_of_row(const CosetParams& p, unsigned long long all, CosetInst* in, uint32_t* row) {
+  const unsigned long long r = blockIdx.x * static_cast<unsigned long long>(kOrderBlock) + threadIdx.x;
+  if (r >= all) return false;
+  uint32_t lo = 0, hi = p.count;
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) / 2;
+    if (p.inst[mid].row_off <= r) lo = mid;
+    else hi = mid;
+  }
+  *in = p.inst[lo];
+  *row = static_cast<uint32_t>(r - in->row_off);
+  return true;
+}
+
+__global__ void __launch_bounds__(kOrderBlock) coset_orbits(CosetParams p, unsigned long long all) {
+  __shared__ uint32_t sum;
+  if (threadIdx.x == 0) sum = 0;
+  __syncthreads();
+  CosetInst in;
+  uint32_t row;
+  uint32_t mine = job_of_row(p, all, &in, &row) ? orbit_of_least(p, in, row) : 0u;
+  mine = __reduce_add_sync(kFullMask, mine);
+  if ((threadIdx.x & 31u) == 0 && mine) atomicAdd(&sum, mine);
+  __syncthreads();
+  if (threadIdx.x == 0) p.order_sums[blockIdx.x] = sum;
+}
+
+__global__ void __launch_bounds__(kOrderBlock) coset_order(CosetParams p, unsigned long long all) {
+  __shared__ uint32_t before, sums[kOrderBlock / 32];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) before = 0;
+  __syncthreads();
+  uint32_t earlier = 0;
+  for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kOrderBlock) earlier += p.order_sums[b];
+  earlier = __reduce_add_sync(kFullMask, earlier);
+  if (lane == 0 && earlier) atomicAdd(&before, earlier);
+  CosetInst in;
+  uint32_t row = 0;
+  const uint32_t mine = job_of_row(p, all, &in, &row) ? orbit_of_least(p, in, row) : 0u;
+  uint32_t upto = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t up = __shfl_up_sync(kFullMask, upto, o);
+    if (lane >= static_cast<uint32_t>(o)) upto += up;
+  }
+  if (lane == 31) sums[warp] = upto;
+  __syncthreads();
+  uint32_t at = before + upto - mine;
+  for (uint32_t w = 0; w < warp; ++w) at += sums[w];
+  for (uint32_t k = 0, x = row; k < mine; ++k) {
+    p.order[at + k] = x;
+    if (k + 1 < mine)
+      x = static_cast<uint32_t>(p.desc[in.desc_off + static_cast<unsigned long long>(x) * in.gens + in.walk]);
+  }
+}
+
 // A table entry in the form the pull uses without unpacking: the byte permute
 // selector of the inner flips in the low half (of the low word; the high
 // word's is it ^ 0x4444), the node's image in the high half.  32-bit words keep
@@ -512,14 +596,11 @@ __global__ void __launch_bounds__(coset_threads<W>(), 1024 / coset_threads<W>())
     // one is worked on: parents differ too much in what they hold for a fixed
     // split (S12, six random generators: 30 % of the warps' time went into
     // waiting at the barrier), and warps that stay close together find each
-    // other's rows in L2 (S13, adjacent transpositions: 54.6 ms, 67.4 ms with
-    // three quarters of the items fixed).  A layer with fewer states than items
-    // skips nearly all of them, which the counter would only slow (S13: 39 ->
-    // 67 us for an empty one): those go round the warps.
+    // other's rows in L2.  A layer with fewer states than items skips nearly all
+    // of them, which the counter would only slow: those go round the warps.
     // 64-bit words: a block is all of a multiprocessor and its warps share a
     // chunk of neighbouring rows, whose parents largely coincide: what one warp
-    // has read the others find in L1.  L2 gives the multiprocessors 5 to 6 TB/s
-    // (bulk copies of whole rows reach no more), which is what such a layer waits for.
+    // has read the others find in L1 (64 % of the sectors on S13 LRX).
     constexpr bool kChunks = sizeof(W) == 8;
     const bool counter = !kChunks && (p.count > 1 || __ldcg(p.counts + d) >= items);
     if (kChunks && threadIdx.x == 0) tickets[(d + 1) & 1u] = 0;
@@ -556,9 +637,12 @@ __global__ void __launch_bounds__(coset_threads<W>(), 1024 / coset_threads<W>())
       const uint32_t unit0 = (item - p.item_prefix[i]) * p.units, all_units = in.rows * kCosetParts;
       // Parents that hold anything, of this lane's unit.
       const uint32_t my_unit = unit0 + (lane & unit_mask);
-      uint32_t parents = 0, own_cur = 0, own_nxt = 0;
+      uint32_t parents = 0, own_cur = 0, own_nxt = 0, place = 0;  // place: row << 3 | part
       if (my_unit < all_units) {
-        const uint32_t row = my_unit / kCosetParts, shift = 8 * (my_unit - row * kCosetParts);
+        uint32_t row = my_unit / kCosetParts;
+        const uint32_t part = my_unit - row * kCosetParts, shift = 8 * part;
+        if (kChunks && in.walk != kNoWalk) row = __ldg(p.order + in.row_off + row);
+        place = (row << 3) | part;
         const unsigned long long* desc = p.desc + in.desc_off + static_cast<unsigned long long>(row) * in.gens;
         for (uint32_t g = lane / p.units; g < in.gens; g += 32u / p.units)
           if (cur_flags[in.row_off + static_cast<uint32_t>(__ldg(desc + g))]) parents |= 1u << g;
@@ -570,7 +654,7 @@ __global__ void __launch_bounds__(coset_threads<W>(), 1024 / coset_threads<W>())
         const uint32_t mask = __shfl_sync(kFullMask, parents, u);
         const uint32_t in_cur = __shfl_sync(kFullMask, own_cur, u), in_nxt = __shfl_sync(kFullMask, own_nxt, u);
         if (!mask && !in_nxt) continue;  // nothing comes in and nothing is to be cleared
-        const uint32_t unit = unit0 + u, row = unit / kCosetParts, part = unit - row * kCosetParts;
+        const uint32_t here = __shfl_sync(kFullMask, place, u), row = here >> 3, part = here & 7u;
         const uint32_t x0 = part * 128u + lane;
         // Lane g holds generator g's descriptor.
         uint32_t from_row = 0, how = 0;  // parent row; slot permutation | outer flips << 16
@@ -1002,7 +1086,7 @@ bool coset_supported(uint32_t n, uint32_t gens) {
 uint64_t coset_job_bytes(const CosetJob& job, uint32_t max_depth) {
   const uint32_t rows = rows_of(embedded(job.n));
   const uint64_t word = coset_wide(job.n) ? 8 : 4, buffers = job.inverse_closed ? 2 : 3;
-  return rows * (buffers * kCosetStride * word + 16 + 8ull * job.gens) + sizeof(CosetInst) + 4 + 16ull * job.gens +
+  return rows * (buffers * kCosetStride * word + 20 + 8ull * job.gens) + sizeof(CosetInst) + 4 + 16ull * job.gens +
          8ull * (max_depth + 2);
 }
 
@@ -1143,6 +1227,7 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   std::vector<uint32_t> prefix(count + 1, 0);
   std::vector<uint8_t> perms;
   unsigned long long rows = 0, descs = 0, visited_rows = 0;
+  bool walks = false;
   for (uint32_t i = 0; i < count; ++i) {
     const CosetJob& j = jobs[i];
     CosetInst& c = inst[i];
@@ -1165,6 +1250,19 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
         }
       if (!(swaps & 1u)) c.same_layer = 1;
     }
+    c.walk = kNoWalk;
+    uint32_t greatest = 2;
+    for (uint32_t g = 0; g < j.gens; ++g) {
+      const uint32_t* s = j.perms + static_cast<size_t>(g) * j.n;
+      uint32_t order = 1;
+      for (uint32_t k = 0; k < j.n; ++k) {
+        uint32_t length = 1;
+        for (uint32_t at = s[k]; at != k; at = s[at]) ++length;
+        order = std::lcm(order, length);
+      }
+      if (wide && order > greatest) greatest = order, c.walk = g;
+    }
+    walks |= c.walk != kNoWalk;
     rows += c.rows;
     descs += static_cast<unsigned long long>(c.rows) * c.gens;
     if (!j.inverse_closed) visited_rows = rows;
@@ -1191,6 +1289,8 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   const size_t cleared = off;
   const size_t o_stamps = take(8ull * stride), o_small = take(16ull * kCosetSmall), o_table = take(table_bytes());
   const size_t o_desc = take(8 * descs);
+  const uint64_t order_blocks = (rows + kOrderBlock - 1) / kOrderBlock;
+  const size_t o_order = take(wide ? 4 * rows : 0), o_order_sums = take(wide ? 4 * order_blocks : 0);
   int rc = memory->arena.ensure(off, true);
   for (int k = 0; k < 3 && !rc && own; ++k)
     if (word_bytes[k]) rc = memory->words[k].ensure(word_bytes[k], true);
@@ -1221,6 +1321,8 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   p.used = reinterpret_cast<uint8_t*>(base + o_used);
   p.table = reinterpret_cast<uint32_t*>(base + o_table);
   p.desc = reinterpret_cast<unsigned long long*>(base + o_desc);
+  p.order = reinterpret_cast<uint32_t*>(base + o_order);
+  p.order_sums = reinterpret_cast<uint32_t*>(base + o_order_sums);
   p.flags[0] = reinterpret_cast<unsigned long long*>(base + o_flags0);
   p.flags[1] = reinterpret_cast<unsigned long long*>(base + o_flags1);
   p.buf[0] = words[0];
@@ -1250,6 +1352,10 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
         std::min<unsigned long long>((descs + kCosetBlock - 1) / kCosetBlock, 8ull * static_cast<uint32_t>(sm_count)));
     if (wide) coset_setup<unsigned long long><<<setup, kCosetBlock, 0, stream>>>(p);
     else coset_setup<uint32_t><<<setup, kCosetBlock, 0, stream>>>(p);
+    if (walks) {
+      coset_orbits<<<static_cast<uint32_t>(order_blocks), kOrderBlock, 0, stream>>>(p, rows);
+      coset_order<<<static_cast<uint32_t>(order_blocks), kOrderBlock, 0, stream>>>(p, rows);
+    }
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) {
@@ -1264,7 +1370,7 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
     ctl.steps = p.report->steps;
     ctl.error = ctl.steps ? p.report->error : static_cast<uint32_t>(ERR_WAIT_LIMIT);  // no report: a barrier gave up
   }
-  out->launches = 2;
+  out->launches = walks ? 4 : 2;
   out->steps = ctl.steps;
   out->fatal = ctl.error;
   // Columns 0 .. steps of the layer table, and the step times.
