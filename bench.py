@@ -8,8 +8,8 @@ Workloads (one step = one pass of the workload):
 * ``s13-lrx`` (default, the headline): the Cayley graph of S13 under L (cyclic
   left shift), R (cyclic right shift) and X (swap of positions 0, 1), full BFS
   from the identity: 13! = 6,227,020,800 states, 79 layers, 18,681,062,400
-  successors, exact Lehmer-rank bitmap.  Every BFS's table is checked against
-  the reference's shipped table.
+  successors, exact bitmap of the rank domain under the default plan.  Every
+  BFS's table is checked against the reference's shipped table.
 * ``s14-lrx``: the same graph on 14 symbols, 14! = 87,178,291,200 states in 92
   layers (peak 4,595,217,203), on one GPU: grouped layers of 24,024 prefix
   groups; checked by its total and the reference's first 24 layers.
@@ -33,6 +33,7 @@ CUDA events on the launching stream over the K steps; ``e2e`` is the same
 metric through the C ABI from host buffers (create -> plan -> run -> tables ->
 destroy, every step, wall clock); ``roofline`` divides algorithmic bytes
 B_alg = 16 N + 32 E p by the summed duration of the layer-expansion launches;
+(searches without frontier lists: the words their layers occupy, `word_bytes`);
 ``cpu_baseline`` is the C oracle (a CPU restatement of the reference's exact
 BFS) on all host cores over a bounded sample of the same workload.
 ``--impl reference`` times that CPU implementation alone (rank 0).
@@ -75,12 +76,12 @@ def coxeter(n):
 
 
 WORKLOADS = {
-    "s13-lrx": dict(n=13, gens=lrx(13), visited="bitmap", dedup="grouped",
+    "s13-lrx": dict(n=13, gens=lrx(13), visited="bitmap", dedup="auto",
                     desc="S13 LRX full BFS (L, R, X from identity; 6,227,020,800 states), exact Lehmer-rank bitmap"),
     "s14-lrx": dict(n=14, gens=lrx(14), visited="bitmap", dedup="auto",
-                    desc="S14 LRX full BFS (87,178,291,200 states, 4.6e9 in the peak layer), exact Lehmer-rank "
-                         "bitmap, grouped layers with 24,024 prefix groups and a memory-bounded spill"),
-    "s13-coxeter": dict(n=13, gens=coxeter(13), visited="bitmap", dedup="grouped",
+                    desc="S14 LRX full BFS (87,178,291,200 states, 4.6e9 in the peak layer), exact bitmap of the "
+                         "rank domain"),
+    "s13-coxeter": dict(n=13, gens=coxeter(13), visited="bitmap", dedup="auto",
                         desc="S13 adjacent transpositions s1..s12 full BFS (6,227,020,800 states), exact bitmap"),
     "s11-lrx-hash": dict(n=11, gens=lrx(11), visited="hash", dedup="atomic",
                          desc="S11 LRX full BFS (39,916,800 states), exact-key open-addressing hash of all visited states"),
@@ -333,6 +334,36 @@ def roofline(b_alg, seconds, kernel, traffic=None, traffic_source=None, **extra)
     return out
 
 
+def whole_search_words(workload, plan):
+    """(words, states per word, bytes per word, kind, kernel) of a search that
+    the default plan runs without frontier lists, None for list layers: coset
+    words of distinct labels, bit rings of 2x2 matrices over a prime field."""
+    if plan["visited"] != "bitmap":
+        return None
+    if "matrix_p" in workload:
+        p = workload["matrix_p"]
+        return ((p - 1) * (p * p - 1), p, 32, "ring",
+                "ring_wave_kernel (unipotent-ring layers; small layers expand_packed)")
+    words = coset_words(workload["n"])
+    return *words, ("coset_small_kernel" if workload["n"] <= 10 else "coset_wave_kernel") + " (coset-word layers)"
+
+
+def coset_words(n):
+    """(words, states per word, bytes per word, kind) of S_n."""
+    per_word = 8 << max(0, min(3, (n - 7) // 2))
+    return max(1, math.factorial(n) // per_word), per_word, 8 if n >= 13 else 4, "coset"
+
+
+def word_bytes(sizes, words, per_word, width, kind):
+    """Bytes a search in words cannot do without: a word that holds a state of a
+    layer is written once, read once as a parent and replaced once.  A layer of s
+    states is taken to lie in words (1 - exp(-s / words)) coset words, and in the
+    fewest rings that hold it (a layer has few determinants)."""
+    if kind == "ring":
+        return int(sum(3 * width * min(s, max(1, s / per_word)) for s in sizes))
+    return int(sum(3 * width * words * -math.expm1(-s / words) for s in sizes))
+
+
 # ---------------------------------------------------------------------------
 # Batched sweep.
 
@@ -408,6 +439,11 @@ def bench_sweep(args, rank, world, local):
             assert gathered == expect, "gathered sweep tables differ from the oracle fixture"
     if rank == 0:
         all_states = sum(map(sum, expect))
+        if args.host_loop:
+            b_alg, kernel = 16 * states + 32 * succ, "batch_expand (layers over frontier lists)"
+        else:
+            b_alg = sum(word_bytes(table, *coset_words(len(g["start"]))[:4]) for g, table in zip(mine, tables))
+            kernel = "coset_wave_kernel (one persistent cooperative launch per wave)"
         line = {"metric": "successors/s", "value": total_succ * args.steps / dev_max, "unit": "successors/s",
                 "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
                 "ms_per_step": dev_max / args.steps * 1e3, "higher_is_better": True,
@@ -421,8 +457,7 @@ def bench_sweep(args, rank, world, local):
                 "wall_ms_per_step": sum(r["seconds"] for r in runs) / len(runs) * 1e3,
                 "e2e": {"value": total_succ / e2e_max, "unit": "successors/s", "h2d_bytes_per_step": h2d,
                         "d2h_bytes_per_step": d2h},
-                "roofline": roofline(16 * states + 32 * succ, dev_s / args.steps,
-                                     "batch_wave (one persistent cooperative launch per wave)", traffic=None),
+                "roofline": roofline(b_alg, dev_s / args.steps, kernel, traffic=None),
                 "waves": runs[0]["waves"], "layer_steps": runs[0]["layer_steps"],
                 "gpu_launches": launches, "clocks": clocks.summary()}
         if world == 1 and not args.no_cpu_baseline:
@@ -656,12 +691,14 @@ def bench_single(args, rank, world, local):
         dist.all_reduce(e2e_t, op=dist.ReduceOp.MAX)
 
     if rank == 0:
-        b_alg = int(16 * states + 32 * succ * probes)
+        words = None if dedup != "auto" or args.host_loop else whole_search_words(w, plan)
+        b_alg = word_bytes(results[0].layer_sizes, *words[:4]) if words else int(16 * states + 32 * succ * probes)
         traffic, source = None, None
         prof = ROOT / "profiles" / f"traffic_{args.workload}.json"
         if prof.exists():
             try:
-                traffic = json.loads(prof.read_text()).get(plan["dedup"], {}).get("dram_bytes_per_bfs")
+                kind = words[3] if words else plan["dedup"]
+                traffic = json.loads(prof.read_text()).get(kind, {}).get("dram_bytes_per_bfs")
                 source = f"ncu capture summarised in profiles/{prof.name}, not measured in this run"
             except Exception:
                 traffic = None
@@ -680,7 +717,8 @@ def bench_single(args, rank, world, local):
             "vs_baseline": None,
             "dtype": "u64",
             "data": "synthetic",
-            "config": {"workload": w["desc"], "visited": plan["visited"], "dedup": plan["dedup"],
+            "config": {"workload": w["desc"], "visited": plan["visited"],
+                       "dedup": f"auto ({words[3]} layers)" if words else plan["dedup"],
                        "planner": plan["planner"], "parallelism": f"replicas{world}" + (
                            " (each GPU runs the whole BFS; the BFS itself is not split)" if world > 1 else ""),
                        "states_per_bfs": states, "successors_per_bfs": succ, "visited_tests_per_bfs": tests,
@@ -696,6 +734,7 @@ def bench_single(args, rank, world, local):
             "e2e": {"value": world * succ / float(e2e_t.item()), "unit": "successors/s",
                     "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
             "roofline": roofline(b_alg, kernel_s,
+                                 words[4] if words else
                                  kernel_names.get(plan["dedup"], "expand_packed (fused layer expansion)"),
                                  traffic=traffic, traffic_source=source,
                                  **({"probes_per_test": round(probes, 4),

@@ -208,7 +208,7 @@ def choose_profile(graph: GraphDefinition, device: int = 0, *, budget_seconds: f
     plans = candidate_plans(graph)
     per_trial = max(1.0, budget_seconds / (2 * len(plans)))
     # Coset-word layers run whole searches only, and a prefix of list layers
-    # says nothing about them (S13 LRX: 35 ms, the fastest list layers 144 ms).
+    # says nothing about them (S13 LRX: 27 ms, the fastest list layers 144 ms).
     # Where a whole search is as cheap as a pilot every candidate runs one; the
     # larger ones keep the default.
     whole = runs_coset_layers(graph, device)
