@@ -119,3 +119,28 @@ def test_a_sweep_of_every_degree_and_width():
         assert sweep.layer_tables() == tables
         with pytest.raises(Exception):
             sweep.run(max_depth=4)
+
+
+def test_rows_by_orbits():
+    """Degree 13 and 14 in one wave, rows ordered by the orbits of a generator:
+    of the full length, of lengths that differ (cycles of 3, 4 and 5), of the
+    rank where no generator has order 3."""
+    from multigpubfs_b200.batch import BatchSweep
+
+    def cycles(n, *lengths):
+        g, at = list(range(n)), 0
+        for k in lengths:
+            g[at:at + k] = g[at + 1:at + k] + g[at:at + 1]
+            at += k
+        return g
+
+    odd = _generators(random.Random(3), 13, 3, "odd")
+    graphs = [G.permutation_graph(gens, list(range(len(gens[0])))) for gens in (
+        [cycles(13, 13)], odd, [cycles(13, 3, 4, 5)], _closed([cycles(14, 14)]), [cycles(14, 5, 9)],
+        _closed([cycles(13, 5, 3), cycles(13, 3, 2)]))]
+    with BatchSweep(graphs) as sweep:
+        st = sweep.run()
+        assert st["complete_instances"] == len(graphs) and st["fatal"] == 0
+        tables = sweep.layer_tables()
+    for g, table in zip(graphs, tables):
+        assert table == P.packed_bfs(g["action"]["generators"], g["start"], max_states=1 << 20)[0]
