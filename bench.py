@@ -452,7 +452,7 @@ def bench_sweep(args, rank, world, local):
                 "config": {"workload": workload_desc("sweep512"), "instances": len(graphs),
                            "states_per_step": all_states, "successors_per_step": total_succ,
                            "parallelism": f"instances split over {world} rank(s) by g|G|" if world > 1 else "1 GPU",
-                           "l2": "per-instance bitmaps and frontiers together exceed L2 (about 0.3 GB per step)"},
+                           "l2": "the instances' word buffers together exceed L2 (about 0.3 GB per step)"},
                 "settled_states_per_s": all_states * args.steps / dev_max,
                 "wall_ms_per_step": sum(r["seconds"] for r in runs) / len(runs) * 1e3,
                 "e2e": {"value": total_succ / e2e_max, "unit": "successors/s", "h2d_bytes_per_step": h2d,
@@ -722,7 +722,9 @@ def bench_single(args, rank, world, local):
                        "planner": plan["planner"], "parallelism": f"replicas{world}" + (
                            " (each GPU runs the whole BFS; the BFS itself is not split)" if world > 1 else ""),
                        "states_per_bfs": states, "successors_per_bfs": succ, "visited_tests_per_bfs": tests,
-                       "l2": "working set larger than L2 (%s)" % (
+                       "l2": ("working set %s than L2 (%%s)" % ("smaller" if words and 2 * words[0] * words[2] < 126 << 20
+                                                                else "larger")) % (
+                           "two word buffers of %d MB" % (words[0] * words[2] >> 20) if words else
                            "bitmap %d MB, frontiers up to several GB" % (plan["bitmap_bits"] // 8 // (1 << 20))
                            if plan["visited"] == "bitmap" else
                            "table of %d slots = %d MB" % (plan["table_slots"],
