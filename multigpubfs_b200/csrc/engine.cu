@@ -2085,6 +2085,7 @@ int Graph::run_device_loop(const void* fn, ExpandParams* pp, size_t smem, uint64
   h.depth = depth0;
   h.capacity = cap;
   h.gens = gens;
+  h.pause_at = static_cast<uint32_t>(list_stop);
   const int visit = visit_kind();
   if ((visit == V_HASH || visit == V_HASHQ) && !(state_bound && table_slots * hash_load / 100 >= state_bound))
     h.table_limit = table_slots * hash_load / 100;
@@ -2355,8 +2356,11 @@ int Graph::run_lists(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, 
   // up front (frontier capacity for every layer, hash table for every state),
   // no limits and no callback.
   const bool limited = limits && (limits->max_seconds > 0 || limits->max_layers || limits->cancel);
-  const uint64_t loop_cap = std::max<uint64_t>(1, plan.capacity);
-  bool device_loop = !host_loop_only && !list_stop && !bucketed && !grouped_mode && !limited && !cb &&
+  // A loop that stops before a layer of list_stop states makes none larger than
+  // that layer can be.
+  const uint64_t loop_cap =
+      std::max<uint64_t>(1, list_stop ? std::min<uint64_t>(plan.capacity, list_stop * gens) : plan.capacity);
+  bool device_loop = !host_loop_only && !bucketed && !grouped_mode && !limited && !cb &&
                      (bitmap_kind(visit) || visit == V_HASH || visit == V_HASHQ) &&
                      2 * (loop_cap + 2) * 8 <= (16ull << 30);
   // The device loop never grows the table: it must hold every state below

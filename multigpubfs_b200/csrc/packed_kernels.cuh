@@ -45,7 +45,8 @@ struct LoopState {
   // pauses (stop 3) before a layer that could take the table past this many
   // states, and the host loop grows it.  0 = the table holds every state.
   unsigned long long table_limit;
-  uint32_t gens, pad;
+  uint32_t gens;
+  uint32_t pause_at;  // the loop pauses (stop 3) before a layer of this many states; 0 = never
 };
 
 struct ExpandParams {
@@ -203,6 +204,7 @@ __device__ __forceinline__ uint32_t loop_step(LoopState* s, Control* c) {
     c->next_count = 0;
     if (d + 1 >= s->max_entries) stop = 3;
     if (s->table_limit && s->visited + produced * s->gens > s->table_limit) stop = 3;
+    if (s->pause_at && produced >= s->pause_at) stop = 3;
   }
   s->stop = stop;
   return stop;

@@ -64,7 +64,8 @@ def _closed(p, matrices):
 
 
 # Six to eight words a ring; determinant 1 only, many at once, and a small
-# group over all of them.
+# group over all of them; long searches that stay below the rings' layers, and
+# one that comes to them late.
 @pytest.mark.parametrize("p,matrices", [
     (163, [(1, 1, 0, 1), (1, 0, 1, 1), (2, 0, 0, 1)]),
     (193, [(1, 1, 0, 1), (1, 0, 1, 1)]),
@@ -73,6 +74,8 @@ def _closed(p, matrices):
     (67, [(3, 1, 4, 7), (5, 2, 0, 9), (0, 1, 11, 0), (2, 0, 0, 1), (6, 6, 1, 3)]),
     (61, [(2, 0, 0, 1), (0, 1, 1, 0)]),
     (37, [(1, 1, 0, 1)]),
+    (127, [(3, 0, 0, 1), (0, 1, 1, 0)]),
+    (113, [(1, 1, 0, 1), (3, 0, 0, 1), (1, 0, 0, 3)]),
 ])
 def test_generator_sets(p, matrices):
     graph = _closed(p, matrices)
