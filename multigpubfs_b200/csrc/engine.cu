@@ -1348,12 +1348,12 @@ int Graph::make_plan(const mgbfs2_plan_request* req, mgbfs2_plan_info* out) {
   // positions in place of the wide hash where the bitmap is small and not much
   // larger than what the generators can reach.
   const uint64_t reach = state_bound ? std::min(state_bound, rank_total) : rank_total;
-  const HalfJob half_job{elements, distinct, gens, nullptr, nullptr, nullptr, inverse_closed, rank_total, reach};
+  const HalfJob half_job{elements, distinct, gens, nullptr, nullptr, perms.data(), inverse_closed, rank_total, reach};
   half_ok = kind == 0 && !lehmer && !use_product && r.dedup == MGBFS2_DEDUP_AUTO && !host_loop_only && !r.capacity &&
             (packed ? visited == MGBFS2_VISITED_BITMAP && bits == 4
                     : r.visited == MGBFS2_VISITED_AUTO && !r.reserve_bytes && rank_total / 64 <= reach) &&
             !r.shards && !r.blocks_per_sm && !r.parents_per_thread && !r.route_chunk && !r.bucket_min_work &&
-            !r.bucket_margin && !learned && half_supported(elements, distinct, gens, rank_total) &&
+            !r.bucket_margin && !learned && half_supported(half_job) &&
             (!orbit_bound || orbit_bound >= rank_total) && 16 * (reach + 2) <= (16ull << 30) &&
             half_bytes(half_job, kWholeDepth) + (rank_total + 63) / 64 * 8 <= budget / 2;
   // Fixed allocations of the plan.

@@ -276,13 +276,31 @@ uint64_t half_entries(uint32_t symbols, uint32_t bits, uint32_t distinct) {
 
 }  // namespace
 
-bool half_supported(uint32_t n, uint32_t distinct, uint32_t gens, uint64_t total) {
-  if (n < 2 || n > 36 || distinct < 1 || distinct > kHalfMaxLabels || !gens || gens > kHalfMaxGens) return false;
-  if (total < 1 || total >= UINT32_MAX) return false;
+// The generators' displacement terms: one for every distinct shift of each.
+static uint32_t half_terms(const HalfJob& job) {
+  uint32_t terms = 0;
+  for (uint32_t g = 0; g < job.gens; ++g) {
+    const uint32_t* s = job.perms + static_cast<size_t>(g) * job.n;
+    uint64_t shifts[2] = {0, 0};  // bit n + s[i] - i
+    for (uint32_t i = 0; i < job.n; ++i) {
+      const uint32_t at = job.n + s[i] - i;
+      shifts[at / 64] |= 1ull << (at % 64);
+    }
+    terms += static_cast<uint32_t>(__builtin_popcountll(shifts[0]) + __builtin_popcountll(shifts[1]));
+  }
+  return terms;
+}
+
+bool half_supported(const HalfJob& job) {
+  const uint32_t n = job.n, distinct = job.distinct;
+  if (n < 2 || n > 36 || distinct < 1 || distinct > kHalfMaxLabels || !job.gens || job.gens > kHalfMaxGens) return false;
+  if (job.total < 1 || job.total >= UINT32_MAX) return false;
   const uint32_t bits = half_code_bits(distinct), half = (n + 1) / 2;
-  // Three-bit halves are indexed as two table lookups of four symbols.
+  // Three-bit halves are indexed as two table lookups of four symbols.  More
+  // terms than a block keeps in shared memory (32 random generators of 24
+  // positions: 570) go to the wide hash; 16 positions cannot have more.
   return n * bits <= 64 && half * bits <= 31 && (bits < 3 || half <= 8) &&
-         half_entries(half, bits, distinct) <= (1ull << kHalfIndexBits);
+         half_entries(half, bits, distinct) <= (1ull << kHalfIndexBits) && half_terms(job) <= kHalfMaxTerms;
 }
 
 uint64_t half_bytes(const HalfJob& job, uint32_t max_layers) {
@@ -293,7 +311,7 @@ uint64_t half_bytes(const HalfJob& job, uint32_t max_layers) {
 
 int half_wave(const HalfJob& job, uint32_t max_layers, int sm_count, cudaStream_t stream, HalfMemory* memory,
               DeviceBuffer* bitmap, DeviceBuffer* front, uint32_t front_bits, HalfResult* out) {
-  if (!half_supported(job.n, job.distinct, job.gens, job.total) || !max_layers) return MGBFS2_INVALID_ARGUMENT;
+  if (!half_supported(job) || !max_layers) return MGBFS2_INVALID_ARGUMENT;
   HalfParams p{};
   p.n = job.n;
   p.distinct = job.distinct;
@@ -325,7 +343,6 @@ int half_wave(const HalfJob& job, uint32_t max_layers, int sm_count, cudaStream_
     }
     begin.push_back(static_cast<uint32_t>(terms.size()));
   }
-  if (terms.size() > kHalfMaxTerms) return MGBFS2_UNSUPPORTED;
   p.total_terms = static_cast<uint32_t>(terms.size());
   const uint32_t tag_bits = 32 - static_cast<uint32_t>(__builtin_clz(job.gens));
   if (job.inverse_closed && job.n * p.bits + tag_bits <= 64) p.gen_shift = job.n * p.bits;

@@ -63,7 +63,8 @@ struct HalfResult {
   double kernel_seconds = 0.0;
 };
 
-bool half_supported(uint32_t n, uint32_t distinct, uint32_t gens, uint64_t total);
+// job.perms: the generators' displacement terms are counted too.
+bool half_supported(const HalfJob& job);
 uint64_t half_bytes(const HalfJob& job, uint32_t max_layers);
 
 // Runs the search with its visited states in `bitmap` (ceil(total / 64) words,

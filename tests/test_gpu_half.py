@@ -88,3 +88,32 @@ def test_the_bitmap_is_the_list_layers(tmp_path):
             e.plan()
             e.resume(tmp_path / name)
             assert e.run().layer_sizes == full.layer_sizes
+
+
+def _terms(gens):
+    """Displacement terms of a generator set: the distinct shifts of each."""
+    return sum(len({x - i for i, x in enumerate(g)}) for g in gens)
+
+
+@pytest.mark.parametrize("case", ["below", "above", "reversals"])
+def test_wide_starts_of_many_generators(case):
+    """Half-rank layers hold 512 displacement terms; the sets on both sides of
+    that (random permutations of 24 positions, all 31 prefix reversals of 32)
+    are searched under the default plan."""
+    if case == "reversals":
+        gens = [list(range(k))[::-1] + list(range(k, 32)) for k in range(2, 33)]
+        start = [1, 1, 1] + [0] * 29
+    else:
+        rng = random.Random(24)
+        gens = [rng.sample(range(24), 24) for _ in range(32)]
+        while case == "below" and _terms(gens) > 512:
+            gens.pop()
+        start = [1] * 4 + [0] * 20
+    assert (_terms(gens) <= 512) == (case == "below") and len(gens) > 16
+    graph = G.permutation_graph(gens, start)
+    lists, last, small, _ = _search(graph, visited="hash")
+    r, current, previous, _ = _search(graph)
+    assert r.complete and r.layer_sizes == lists.layer_sizes
+    assert previous == small
+    if r.layer_sizes[-1] <= 1000:
+        assert current == last
