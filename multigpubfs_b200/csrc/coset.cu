@@ -1,6 +1,7 @@
 // Coset-word layers (see coset.h for the coordinates): tables, the persistent
 // wave kernel, the read-out of the deepest layer, and their host side.
 #include "coset.h"
+#include "search_end.h"
 
 #include <algorithm>
 #include <cstring>
@@ -1094,16 +1095,13 @@ uint64_t coset_fixed_bytes(uint32_t max_depth) {
   return table_bytes() + kSlotPerms + 16ull * kCosetSmall + 20ull * (max_depth + 2) + 32 * 256;
 }
 
-// Layer tables (count x cols sizes, 0 past the deepest) and step times.
+// Layer tables (count x end.columns sizes) and step times.
 static void read_layers(const std::vector<unsigned long long>& counts, const std::vector<unsigned long long>& stamps,
-                        uint32_t count, uint32_t cols, uint32_t max_depth, CosetResult* out) {
-  out->layers.assign(count, {});
+                        uint32_t count, const SearchEnd& end, uint32_t max_depth, CosetResult* out) {
+  const uint32_t cols = end.fatal ? 1 : end.columns;
+  out->layers = layer_tables(counts.data(), count, end);
   out->overflow.assign(count, 0);
-  for (uint32_t i = 0; i < count; ++i) {
-    const unsigned long long* row = counts.data() + static_cast<size_t>(i) * cols;
-    for (uint32_t d = 0; d < cols && row[d]; ++d) out->layers[i].push_back(row[d]);
-    out->overflow[i] = out->layers[i].size() > max_depth;
-  }
+  for (uint32_t i = 0; i < count; ++i) out->overflow[i] = out->layers[i].size() > max_depth;
   out->step_seconds.clear();
   for (uint32_t d = 0; d + 1 < cols; ++d) out->step_seconds.push_back(static_cast<double>(stamps[d + 1] - stamps[d]) * 1e-9);
   out->kernel_seconds = cols > 1 ? static_cast<double>(stamps[cols - 1] - stamps[0]) * 1e-9 : 0.0;
@@ -1160,8 +1158,9 @@ static int coset_small(const CosetJob& job, uint32_t max_depth, uint32_t units, 
   MG_CHECK_COSET(cudaStreamSynchronize(stream));
   out->launches = 1;
   out->steps = p.report->steps;
-  out->fatal = out->steps ? p.report->error : static_cast<uint32_t>(ERR_WAIT_LIMIT);  // no report: a barrier gave up
-  const uint32_t cols = std::min(out->steps + 1, stride);
+  const SearchEnd end = search_end(out->steps, p.report->error, stride, ERR_WAIT_LIMIT);
+  out->fatal = end.fatal;
+  const uint32_t cols = end.columns;
   std::vector<unsigned long long> counts(cols, 0), stamps(cols, 0);
   if (cols <= kReportLayers) {
     std::memcpy(counts.data(), p.report->counts, 8ull * cols);
@@ -1171,8 +1170,7 @@ static int coset_small(const CosetJob& job, uint32_t max_depth, uint32_t units, 
     MG_CHECK_COSET(cudaMemcpyAsync(stamps.data(), p.stamps, 8ull * cols, cudaMemcpyDeviceToHost, stream));
     MG_CHECK_COSET(cudaStreamSynchronize(stream));
   }
-  if (out->fatal) counts.assign(1, 1);
-  read_layers(counts, stamps, 1, static_cast<uint32_t>(counts.size()), max_depth, out);
+  read_layers(counts, stamps, 1, end, max_depth, out);
   if (out->fatal || out->overflow[0]) return MGBFS2_OK;
   out->previous_small.assign(p.report->previous, p.report->previous + p.report->previous_count);
   const uint64_t deepest = out->layers[0].back();
@@ -1368,13 +1366,14 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   if (e != cudaSuccess) return cuda_status(e);
   if (p.report) {
     ctl.steps = p.report->steps;
-    ctl.error = ctl.steps ? p.report->error : static_cast<uint32_t>(ERR_WAIT_LIMIT);  // no report: a barrier gave up
+    ctl.error = p.report->error;
   }
+  const SearchEnd end = search_end(ctl.steps, ctl.error, stride, ERR_WAIT_LIMIT);
   out->launches = walks ? 4 : 2;
   out->steps = ctl.steps;
-  out->fatal = ctl.error;
+  out->fatal = end.fatal;
   // Columns 0 .. steps of the layer table, and the step times.
-  const uint32_t cols = std::min(ctl.steps + 1, stride);
+  const uint32_t cols = end.columns;
   std::vector<unsigned long long> stamps(cols), counts(static_cast<size_t>(count) * cols);
   if (p.report && cols <= kReportLayers) {
     std::memcpy(counts.data(), p.report->counts, 8ull * cols);
@@ -1385,7 +1384,7 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
     MG_CHECK_COSET(cudaMemcpyAsync(stamps.data(), p.stamps, 8ull * cols, cudaMemcpyDeviceToHost, stream));
     MG_CHECK_COSET(cudaStreamSynchronize(stream));
   }
-  read_layers(counts, stamps, count, cols, max_depth, out);
+  read_layers(counts, stamps, count, end, max_depth, out);
   if (!collect || out->fatal || out->overflow[0]) return MGBFS2_OK;
   const CosetReport& r = *p.report;
   out->previous_small.assign(r.previous, r.previous + r.previous_count);

@@ -1,6 +1,7 @@
 // Half-rank layers (see half.h): tables, the persistent wave kernel and its
 // host side.
 #include "half.h"
+#include "search_end.h"
 
 #include <algorithm>
 #include <cstring>
@@ -420,8 +421,9 @@ int half_wave(const HalfJob& job, uint32_t max_layers, int sm_count, cudaStream_
   MG_CHECK_HALF(cudaLaunchCooperativeKernel(wave, dim3(blocks), dim3(kHalfBlock), args, 0, stream));
   MG_CHECK_HALF(cudaStreamSynchronize(stream));
   out->launches = 2;
-  out->fatal = report->steps ? report->error : static_cast<uint32_t>(ERR_WAIT_LIMIT);  // no report: a barrier gave up
-  const uint32_t steps = report->steps, cols = std::min(steps + 1, stride);
+  const SearchEnd end = search_end(report->steps, report->error, stride, ERR_WAIT_LIMIT);
+  out->fatal = end.fatal;
+  const uint32_t cols = end.columns;
   std::vector<unsigned long long> counts(cols), stamps(cols);
   if (cols <= kHalfReportLayers) {
     std::memcpy(counts.data(), report->counts, 8ull * cols);

@@ -1,6 +1,7 @@
 // Unipotent-ring layers (see ring.h): seeding from frontier lists, the persistent
 // wave kernel and its host side.
 #include "ring.h"
+#include "search_end.h"
 
 #include <algorithm>
 #include <cstring>
@@ -484,8 +485,9 @@ int ring_wave(uint32_t p, uint32_t bits, uint32_t gens, const uint32_t* coef, co
                                             dim3(kRingBlock), args, 0, stream));
   ++out->launches;
   MG_CHECK_RING(cudaStreamSynchronize(stream));
-  out->fatal = report->steps ? report->error : static_cast<uint32_t>(ERR_WAIT_LIMIT);  // no report: a barrier gave up
-  const uint32_t steps = report->steps, cols = std::min(steps + 1, stride);
+  const SearchEnd end = search_end(report->steps, report->error, stride, ERR_WAIT_LIMIT);
+  out->fatal = end.fatal;
+  const uint32_t steps = report->steps, cols = end.columns;
   std::vector<unsigned long long> counts(cols), stamps(cols);
   if (cols <= kRingReportLayers) {
     std::memcpy(counts.data(), report->counts, 8ull * cols);

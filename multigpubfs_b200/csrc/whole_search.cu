@@ -24,6 +24,23 @@ using Clock = std::chrono::steady_clock;
 // than its edges; small orbits, p = 127: 129 layers in 1.6 ms), unless there are so few nodes
 // that the pass costs no more than a launch (p = 67: 10 us a layer).
 constexpr uint64_t kRingShare = 64, kRingFewNodes = 1ull << 20;
+
+// The handle of a packed search that knows its start alone: one that is about
+// to begin, or one that failed.
+int start_only(Graph* g) {
+  g->layer_sizes.assign(1, 1);
+  g->layer_seconds.clear();
+  g->front_grouped = false;
+  for (int i = 0; i < 2; ++i) {
+    g->small_layer[i].clear();
+    g->small_depth[i] = UINT32_MAX;
+  }
+  g->keep_small(0, std::vector<uint64_t>(1, g->start_word));
+  g->last_count = 1;
+  if (int rc = g->front.ensure(16)) return rc;
+  MG_CHECK(cudaMemcpyAsync(g->front.ptr, &g->start_word, 8, cudaMemcpyHostToDevice, g->stream));
+  return MGBFS2_OK;
+}
 }  // namespace
 
 // A whole search in coset-word layers, from the identity: the layer sizes do
@@ -56,11 +73,13 @@ int Graph::coset_run(mgbfs2_status* status) {
     small_layer[i].clear();
     small_depth[i] = UINT32_MAX;
   }
-  if (!r.fatal) {
+  if (r.fatal) {
+    if (int rc = start_only(this)) return rc;
+  } else {
     if (deepest && layer_sizes[deepest - 1] < kCosetSmall) keep_small(deepest - 1, std::move(r.previous_small));
     if (layer_sizes[deepest] < kCosetSmall) keep_small(deepest, std::move(r.deepest_small));
+    last_count = layer_sizes[deepest];
   }
-  last_count = r.fatal ? 0 : layer_sizes[deepest];
   launches = r.launches;
   st.complete = r.fatal == 0;
   st.reason = r.fatal ? MGBFS2_REASON_RESOURCE : MGBFS2_REASON_FRONTIER_EXHAUSTED;
@@ -99,19 +118,9 @@ int Graph::ring_run(mgbfs2_status* status) {
       return rc;
     }
   } else {
-    layer_sizes.assign(1, 1);
-    layer_seconds.clear();
-    front_grouped = false;
-    for (int i = 0; i < 2; ++i) {
-      small_layer[i].clear();
-      small_depth[i] = UINT32_MAX;
-    }
-    keep_small(0, std::vector<uint64_t>(1, start_word));
-    last_count = 1;
     launches = 0;
     st.states = st.layers = 1;
-    if (int rc = front.ensure(16)) return rc;
-    MG_CHECK(cudaMemcpyAsync(front.ptr, &start_word, 8, cudaMemcpyHostToDevice, stream));
+    if (int rc = start_only(this)) return rc;
   }
   if (!ring) {
     ring = new RingMemory();
@@ -193,7 +202,9 @@ int Graph::half_run(mgbfs2_status* status) {
     half_rows[i].clear();
   }
   const auto symbol = [&](uint64_t w, uint32_t i) { return (w >> (r.bits * i)) & ((1ull << r.bits) - 1ull); };
-  if (packed) {
+  if (packed && r.fatal) {
+    if (int rc = start_only(this)) return rc;
+  } else if (packed) {
     const auto words = [&](const std::vector<uint64_t>& states) {
       std::vector<uint64_t> out;
       for (uint64_t w : states) {
@@ -205,8 +216,10 @@ int Graph::half_run(mgbfs2_status* status) {
     };
     if (deepest && layer_sizes[deepest - 1] < kHalfSmall) keep_small(deepest - 1, words(r.previous));
     if (layer_sizes[deepest] < kHalfSmall) keep_small(deepest, words(r.deepest));
+    last_count = layer_sizes[deepest];
   } else {
     half_done = true;
+    last_count = layer_sizes[deepest];
     const auto rows = [&](const std::vector<uint64_t>& states, std::vector<std::vector<int64_t>>* out) {
       for (uint64_t w : states) {
         std::vector<int64_t> row(elements);
@@ -216,8 +229,8 @@ int Graph::half_run(mgbfs2_status* status) {
     };
     rows(r.deepest, &half_rows[0]);
     rows(r.previous, &half_rows[1]);
+    if (r.fatal) half_rows[0].assign(1, start);
   }
-  last_count = r.fatal ? 0 : layer_sizes[deepest];
   launches = r.launches;
   st.complete = r.fatal == 0;
   st.reason = r.fatal ? MGBFS2_REASON_RESOURCE : MGBFS2_REASON_FRONTIER_EXHAUSTED;
