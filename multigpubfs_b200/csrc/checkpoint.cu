@@ -108,6 +108,43 @@ struct Pinned {
 
 }  // namespace
 
+// A complete search without frontier lists left no rank bitmap: list layers
+// make it, and the deepest layer with its tags.  List layers need more memory
+// than the search did; where they do not come to the same table the handle
+// keeps what the search gave it.
+static int make_bitmap(Graph* g) {
+  DeviceBuffer front = g->front;
+  g->front = DeviceBuffer();
+  g->front.stream = g->stream;
+  const std::vector<uint64_t> sizes = g->layer_sizes;
+  const std::vector<double> seconds = g->layer_seconds;
+  const std::vector<uint64_t> small[2] = {g->small_layer[0], g->small_layer[1]};
+  const uint32_t depth[2] = {g->small_depth[0], g->small_depth[1]};
+  const uint64_t count = g->last_count;
+  const auto launches = g->launches;
+  mgbfs2_status st{};
+  int rc = g->run_lists(nullptr, nullptr, nullptr, &st);
+  if (!rc && st.fatal) rc = MGBFS2_CAPACITY;
+  if (!rc && (!st.complete || g->layer_sizes != sizes)) rc = MGBFS2_STATE;
+  g->layer_seconds = seconds;
+  g->launches = launches;
+  if (!rc) {
+    front.free();
+    return MGBFS2_OK;
+  }
+  g->front.free();
+  g->front = front;
+  g->front_grouped = false;
+  g->layer_sizes = sizes;
+  for (int i = 0; i < 2; ++i) {
+    g->small_layer[i] = small[i];
+    g->small_depth[i] = depth[i];
+  }
+  g->last_count = count;
+  g->no_bitmap = true;
+  return rc;
+}
+
 int Graph::write_checkpoint(const char* path) {
   if (!path) return MGBFS2_INVALID_ARGUMENT;
   if (!planned || !packed || layer_sizes.empty()) return MGBFS2_STATE;
@@ -116,8 +153,7 @@ int Graph::write_checkpoint(const char* path) {
   MG_CHECK(cudaSetDevice(device));
   MG_CHECK(cudaStreamSynchronize(stream));
   if (no_bitmap) {
-    // A complete search without frontier lists left no rank bitmap.
-    if (int rc = run_lists(nullptr, nullptr, nullptr, nullptr)) return rc;
+    if (int rc = make_bitmap(this)) return rc;
   }
   if (front_grouped) {
     if (int rc = gather_front(last_count)) return rc;
@@ -217,6 +253,7 @@ int Graph::read_checkpoint(const char* path) {
     small_depth[i] = h.small_depth[i];
   }
   last_count = h.frontier;
+  no_bitmap = false;
   resume_pending = true;
   return MGBFS2_OK;
 }

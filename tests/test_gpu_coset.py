@@ -144,3 +144,32 @@ def test_rows_by_orbits():
         tables = sweep.layer_tables()
     for g, table in zip(graphs, tables):
         assert table == P.packed_bfs(g["action"]["generators"], g["start"], max_states=1 << 20)[0]
+
+
+def test_a_checkpoint_that_list_layers_cannot_make(tmp_path):
+    """Coset words fit a budget of 96 MB that the list layers of the same search
+    do not: the search completes, its checkpoint is refused, and the handle
+    keeps the table and the states."""
+    import torch
+    from multigpubfs_b200 import GraphDefinition, native
+    from multigpubfs_b200.engine import NativeGraph
+    rng = random.Random(11)
+    graph = GraphDefinition.from_dict(G.permutation_graph(_closed(_generators(rng, 11, 4, "any")), list(range(11))))
+    with NativeGraph(graph) as e:
+        e.plan()
+        want = e.run()
+        words, samples = sorted(e.frontier_words().tolist()), (e.sample(0), e.sample(1))
+        assert max(want.layer_sizes) > 6 << 20  # more than (96 MB - the bitmap) / 16 bytes
+        native.trim_memory(0)
+        torch.cuda.empty_cache()
+        free, _ = torch.cuda.mem_get_info()
+        e.plan(reserve_bytes=free - (96 << 20))
+        r = e.run()
+        assert r.complete and r.layer_sizes == want.layer_sizes
+        path = tmp_path / "refused.bin"
+        with pytest.raises(native.NativeError):
+            e.checkpoint(path)
+        assert not path.exists()
+        assert e.layer_table()[0] == want.layer_sizes
+        assert sorted(e.frontier_words().tolist()) == words
+        assert (e.sample(0), e.sample(1)) == samples
