@@ -370,6 +370,7 @@ int half_wave(const HalfJob& job, uint32_t max_layers, int sm_count, cudaStream_
   const size_t o_counts = take(8ull * stride), o_ctl = take(sizeof(HalfCtl));
   const size_t cleared = off;
   const size_t o_stamps = take(8ull * stride), o_before = take(4ull * p.entries[0]), o_within = take(4ull * p.entries[1]);
+  memory->deepest = nullptr;
   int rc = memory->arena.ensure(off, true);
   for (DeviceBuffer& b : memory->list)
     if (!rc) rc = b.ensure((job.capacity + 2) * 8, true);
@@ -445,6 +446,9 @@ int half_wave(const HalfJob& job, uint32_t max_layers, int sm_count, cudaStream_
   out->overflow = out->layers.size() > max_layers;
   if (out->overflow) return MGBFS2_OK;
   const uint64_t deepest = out->layers.back(), last = out->layers.size() - 1;
+  memory->deepest = reinterpret_cast<const uint64_t*>(p.list[last & 1]);
+  memory->key_mask = p.gen_shift ? (1ull << p.gen_shift) - 1ull : ~0ull;
+  memory->bits = p.bits;
   out->deepest.assign(report->deepest, report->deepest + std::min<uint64_t>(deepest, kHalfSmall));
   if (last && out->layers[last - 1] < kHalfSmall)
     out->previous.assign(report->previous, report->previous + out->layers[last - 1]);

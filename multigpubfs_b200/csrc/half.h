@@ -27,10 +27,14 @@ constexpr uint32_t kHalfIndexBits = 21;  // table entries of a half
 struct HalfMemory {
   DeviceBuffer arena, list[2];
   void* report = nullptr;  // pinned, from pinned_take
+  const uint64_t* deepest = nullptr;  // the last search's deepest layer, in one of the lists
+  uint64_t key_mask = 0;              // its words without their tags
+  uint32_t bits = 0;                  // bits a symbol
   void set_stream(cudaStream_t s) {
     arena.stream = list[0].stream = list[1].stream = s;
   }
   void free() {
+    deepest = nullptr;
     arena.free();
     for (DeviceBuffer& b : list) b.free();
   }

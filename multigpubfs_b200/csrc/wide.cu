@@ -17,6 +17,7 @@
 #include <cstring>
 
 #include "engine.h"
+#include "half.h"
 
 namespace mgbfs2 {
 
@@ -373,14 +374,25 @@ int Graph::wide_run(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, v
 }
 
 int Graph::wide_sample(uint32_t which, int64_t* out, size_t cap_rows, size_t* rows) {
-  if (half_done) {  // the last run was in half-rank layers: their rows are kept on the host
-    const auto& kept = half_rows[which];
-    const uint64_t n = std::min<uint64_t>(kept.size(), cap_rows);
-    std::vector<std::vector<int64_t>> sorted(kept.begin(), kept.begin() + static_cast<std::ptrdiff_t>(n));
-    std::sort(sorted.begin(), sorted.end());
-    for (uint64_t r = 0; r < n; ++r)
-      if (out) std::memcpy(out + r * elements, sorted[r].data(), elements * sizeof(int64_t));
-    *rows = n;
+  if (half_done) {
+    // The last run was in half-rank layers: the host has up to kHalfSmall rows
+    // of each layer, the device the whole deepest one.
+    std::vector<std::vector<int64_t>> decoded = half_rows[which];
+    if (which == 0 && decoded.size() < std::min<uint64_t>(last_count, cap_rows) && half && half->deepest) {
+      std::vector<uint64_t> words(std::min<uint64_t>(last_count, cap_rows));
+      if (cudaMemcpyAsync(words.data(), half->deepest, words.size() * 8, cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+          cudaStreamSynchronize(stream) != cudaSuccess)
+        return MGBFS2_CUDA_BASE;
+      decoded.assign(words.size(), std::vector<int64_t>(elements));
+      for (size_t r = 0; r < words.size(); ++r)
+        for (uint32_t i = 0; i < elements; ++i)
+          decoded[r][i] = labels[((words[r] & half->key_mask) >> (half->bits * i)) & ((1ull << half->bits) - 1)];
+    }
+    decoded.resize(std::min<uint64_t>(decoded.size(), cap_rows));
+    std::sort(decoded.begin(), decoded.end());
+    for (size_t r = 0; r < decoded.size(); ++r)
+      if (out) std::memcpy(out + r * elements, decoded[r].data(), elements * sizeof(int64_t));
+    *rows = decoded.size();
     return MGBFS2_OK;
   }
   WideState& w = *wide;

@@ -117,3 +117,29 @@ def test_wide_starts_of_many_generators(case):
     assert previous == small
     if r.layer_sizes[-1] <= 1000:
         assert current == last
+
+
+@pytest.mark.parametrize("limit", [1, 999, 1000, 1001, 1820, 5000])
+def test_samples_of_a_large_deepest_layer(limit):
+    """Star transpositions on 20 positions, four of them marked: 1,820 states
+    in the deepest layer, more than the rows a search copies to the host."""
+    from multigpubfs_b200 import GraphDefinition
+    from multigpubfs_b200.engine import NativeGraph
+    n, start = 20, [7] * 4 + [-3] * 16
+    gens = []
+    for i in range(1, n):
+        g = list(range(n))
+        g[0], g[i] = i, 0
+        gens.append(g)
+    graph = GraphDefinition.from_dict(G.permutation_graph(gens, start))
+    with NativeGraph(graph) as e:
+        e.plan(visited="hash")
+        whole = e.run()
+        rows = e.sample(0, 5000)
+    with NativeGraph(graph) as e:
+        e.plan()
+        r = e.run()
+        got = e.sample(0, limit)
+    assert r.layer_sizes == whole.layer_sizes and len(rows) == r.layer_sizes[-1] == 1820
+    assert len(got) == min(limit, 1820) and got == sorted(got)
+    assert len({tuple(x) for x in got}) == len(got) and {tuple(x) for x in got} <= {tuple(x) for x in rows}
