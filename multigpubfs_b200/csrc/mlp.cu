@@ -155,7 +155,11 @@ __global__ void __cluster_dims__(kGradCluster, 1, 1) __launch_bounds__(kGradBloc
       for (uint32_t r = 0; r < kGradPer; ++r) a[r] = fmaf(w, s.x[row0 + r][i], a[r]);
     }
 #pragma unroll
-    for (uint32_t r = 0; r < kGradPer; ++r) s.h1[row0 + r][unit] = fmaxf(a[r], 0.f);
+    for (uint32_t r = 0; r < kGradPer; ++r) {
+      const float h = fmaxf(a[r], 0.f);
+      s.h1[row0 + r][unit] = h;
+      odd = odd || !isfinite(h);  // overflowed from finite inputs
+    }
     __syncthreads();
 #pragma unroll
     for (uint32_t r = 0; r < kGradPer; ++r) a[r] = s.b2[unit];

@@ -233,3 +233,43 @@ def test_loss_grad_leaves_out_products_with_zero():
     assert lib.mgbfs2_mlp_loss_grad(inputs, dev[0].data_ptr(), dev[1].data_ptr(), dev[2].data_ptr(), 1.0, 1.0, rows,
                                     grad.data_ptr(), loss.data_ptr(), native.stream_handle()) == 0
     assert bool(torch.isfinite(grad).all()) and bool(torch.isfinite(loss).all())
+
+
+def _loss_grad(params, x, t, weights, inputs):
+    import torch
+    from multigpubfs_b200 import native
+    lib = native.require_device()
+    dev = [torch.tensor(a, device="cuda") for a in (params, x, t)]
+    grad, loss = torch.zeros(len(params), device="cuda"), torch.zeros(1, device="cuda")
+    assert lib.mgbfs2_mlp_loss_grad(inputs, dev[0].data_ptr(), dev[1].data_ptr(), dev[2].data_ptr(), *weights, len(x),
+                                    grad.data_ptr(), loss.data_ptr(), native.stream_handle()) == 0
+    return grad.cpu().numpy().astype(np.float64), float(loss.item())
+
+
+def test_loss_grad_leaves_out_overflowed_units_behind_a_zero():
+    """A row whose first layer overflows to infinity from finite inputs and whose
+    second layer is off: its products with a zero derivative are left out.
+    Against float64, where nothing overflows; tolerance as for the tiles."""
+    from multigpubfs_b200 import native
+    inputs, rows = 4, 40
+    rng = np.random.default_rng(5)
+    params = rng.normal(0.0, 0.3, int(native.require_device().mgbfs2_mlp_param_count(inputs))).astype(np.float32)
+    w1, b1, w2, b2, w3, b3 = M.split(params, inputs)
+    w1[:, 2], w2[:] = 10.0, -np.abs(w2)
+    params = np.concatenate([a.ravel() for a in (w1, b1, w2, b2, w3, b3)]).astype(np.float32)
+    x = rng.normal(size=(rows, inputs)).astype(np.float32)
+    x[7, 2] = 3e38
+    t = rng.normal(size=(rows, 2)).astype(np.float32)
+    got, loss = _loss_grad(params, x, t, (1.0, 0.5), inputs)
+    h1, on1 = _fp32_units(w1, b1, x)
+    _, on2 = _fp32_units(w2, b2, h1)
+    assert np.isinf(h1[7]).all() and not on2[7].any() and on2.any()
+    y64, (x64, a1, _, a2, _) = M.forward(params.astype(np.float64), x, inputs)
+    e = y64 - t
+    dy = 2.0 / rows * np.array([1.0, 0.5]) * e
+    d2 = (dy @ w3) * on2
+    d1 = (d2 @ w2) * on1
+    grad64 = np.concatenate([(d1.T @ x64).ravel(), d1.sum(0), (d2.T @ (a1 * on1)).ravel(), d2.sum(0),
+                             (dy.T @ (a2 * on2)).ravel(), dy.sum(0)])
+    assert abs(loss - float((np.array([1.0, 0.5]) * e * e).sum() / rows)) <= 2e-6 * (1.0 + abs(loss))
+    assert np.abs(got - grad64).max() <= 2e-6 * (1.0 + np.abs(grad64).max())
