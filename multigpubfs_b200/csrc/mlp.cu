@@ -185,10 +185,10 @@ __global__ void __cluster_dims__(kGradCluster, 1, 1) __launch_bounds__(kGradBloc
       y += __shfl_xor_sync(kFullMask, y, 2);
       const bool valid = base + row < batch;
       const float e = valid ? y - target[(base + row) * kOut + out] : 0.f, w = out ? w1 : w0;
-      const float dy = scale * w * e;
+      const float dy = valid ? scale * w * e : 0.f;  // a row past the batch is 0 under any weight
       if (part == 0) {
         s.dy[row][out] = dy;
-        local_loss += w * e * e / static_cast<float>(batch);
+        if (valid) local_loss += w * e * e / static_cast<float>(batch);
         if (out) gb31 += dy;
         else gb30 += dy;
       }

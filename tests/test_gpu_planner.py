@@ -273,3 +273,15 @@ def test_loss_grad_leaves_out_overflowed_units_behind_a_zero():
                              (dy.T @ (a2 * on2)).ravel(), dy.sum(0)])
     assert abs(loss - float((np.array([1.0, 0.5]) * e * e).sum() / rows)) <= 2e-6 * (1.0 + abs(loss))
     assert np.abs(got - grad64).max() <= 2e-6 * (1.0 + np.abs(grad64).max())
+
+
+def test_rows_past_the_batch_are_zero_under_an_infinite_weight():
+    """One row, 31 rows of padding in its tile: the weighted error is infinite,
+    of the sign of the output's error, and not NaN from the padding."""
+    from multigpubfs_b200 import native
+    rng = np.random.default_rng(6)
+    params = rng.normal(0.0, 0.3, int(native.require_device().mgbfs2_mlp_param_count(4))).astype(np.float32)
+    x = rng.normal(size=(1, 4)).astype(np.float32)
+    t = np.array([[0.25, 50.0]], dtype=np.float32)  # the second output lies far below
+    got, loss = _loss_grad(params, x, t, (1.0, float("inf")), 4)
+    assert got[-1] == -np.inf and np.isfinite(got[-2]) and loss == np.inf
