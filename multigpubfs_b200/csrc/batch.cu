@@ -40,6 +40,7 @@
 #include "../../include/mgbfs2.h"
 #include "coset.h"
 #include "engine.h"
+#include "search_end.h"
 
 #define MG_CHECK_BATCH(expr)                          \
   do {                                                \
@@ -1125,8 +1126,17 @@ int mgbfs2_batch_run(mgbfs2_batch* batch, const mgbfs2_batch_options* options, m
       else coset = false;
       if (!coset) later.resize(later.size() - (wave.size() - same.size()));
     }
-    rc = coset ? run_coset_wave(b, wave, max_depth, &st, &kernel_seconds)
-               : run_wave(b, wave, caps, pool, max_depth, blocks_per_sm, tile_ppt, loop, &st, &kernel_seconds);
+    if (coset) {
+      rc = run_coset_wave(b, wave, max_depth, &st, &kernel_seconds);
+      if (lists_instead(rc)) {
+        cudaGetLastError();
+        caps.clear();
+        for (uint32_t i : wave) caps.push_back(cap[i]);
+        coset = false;
+      }
+    }
+    if (!coset)
+      rc = run_wave(b, wave, caps, pool, max_depth, blocks_per_sm, tile_ppt, loop, &st, &kernel_seconds);
     ++st.waves;
     for (uint32_t i : wave) {
       if (b->inst[i].status == INST_OVERFLOW) {

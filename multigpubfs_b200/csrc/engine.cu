@@ -29,6 +29,7 @@
 #include "half.h"
 #include "packed_kernels.cuh"
 #include "ring.h"
+#include "search_end.h"
 
 namespace mgbfs2 {
 
@@ -2230,10 +2231,12 @@ int Graph::run(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, void* 
   MG_CHECK(cudaSetDevice(device));
   const bool limited = limits && (limits->max_seconds > 0 || limits->max_layers || limits->cancel);
   half_done = false;
-  if (!limited && !cb && !resume_pending) {
-    if (half_ok) return half_run(status);
-    if (coset_ok) return coset_run(status);
-    if (ring_ok) return ring_run(status);
+  if (!limited && !cb && !resume_pending && (half_ok || coset_ok || ring_ok)) {
+    const int rc = half_ok ? half_run(status) : coset_ok ? coset_run(status) : ring_run(status);
+    if (!lists_instead(rc)) return rc;
+    cudaGetLastError();
+    if (coset) coset->free();
+    if (ring) ring->free();
   }
   if (!packed) {
     if (half) half->free();

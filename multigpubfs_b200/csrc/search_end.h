@@ -7,7 +7,17 @@
 #include <cstdint>
 #include <vector>
 
+#include "../../include/mgbfs2.h"
+
 namespace mgbfs2 {
+
+// Whether list layers run a search that a form without them returned `rc` for:
+// its buffers did not fit (the plan looked at the memory, but takes none of
+// theirs), or its grid cannot be resident as a whole.
+constexpr int kCooperativeTooLarge = MGBFS2_CUDA_BASE + 720, kNotSupported = MGBFS2_CUDA_BASE + 801;
+constexpr bool lists_instead(int rc) {
+  return rc == MGBFS2_OUT_OF_MEMORY || rc == MGBFS2_UNSUPPORTED || rc == kCooperativeTooLarge || rc == kNotSupported;
+}
 
 struct SearchEnd {
   uint32_t fatal;    // device ERR_* bits

@@ -7,8 +7,13 @@
 #include "engine.h"
 #include "half.h"
 #include "ring.h"
+#include "search_end.h"
 
 namespace mgbfs2 {
+
+static_assert(kCooperativeTooLarge == MGBFS2_CUDA_BASE + cudaErrorCooperativeLaunchTooLarge &&
+                  kNotSupported == MGBFS2_CUDA_BASE + cudaErrorNotSupported,
+              "the codes that cuda_status makes of a cooperative launch's errors");
 
 #define MG_CHECK(expr)                         \
   do {                                         \

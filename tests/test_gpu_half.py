@@ -143,3 +143,29 @@ def test_samples_of_a_large_deepest_layer(limit):
     assert r.layer_sizes == whole.layer_sizes and len(rows) == r.layer_sizes[-1] == 1820
     assert len(got) == min(limit, 1820) and got == sorted(got)
     assert len({tuple(x) for x in got}) == len(got) and {tuple(x) for x in got} <= {tuple(x) for x in rows}
+
+
+def test_lists_that_do_not_fit_leave_the_search_to_the_hash():
+    """C(30, 15) = 155 M arrangements bound the layers of a shift's 30 states:
+    with 1.5 GB left on the device when the search runs, half-rank layers do not
+    get their two lists of 1.24 GB, and the wide hash needs a few MB."""
+    import torch
+    from multigpubfs_b200 import GraphDefinition, native
+    from multigpubfs_b200.engine import NativeGraph
+    shift = list(range(1, 30)) + [0]
+    graph = GraphDefinition.from_dict(G.permutation_graph([shift, [29] + list(range(29))], [1] * 15 + [0] * 15))
+    native.trim_memory(0)
+    torch.cuda.empty_cache()
+    with NativeGraph(graph) as e:
+        e.plan()
+        free, _ = torch.cuda.mem_get_info()
+        hold = torch.empty(free - (1536 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            r = e.run()
+            rows = e.sample(0)
+        finally:
+            del hold
+            torch.cuda.empty_cache()
+        assert r.complete and r.layer_sizes == [1] + [2] * 14 + [1]
+        assert rows == [[0] * 15 + [1] * 15]
+        assert e.run().layer_sizes == r.layer_sizes and e.sample(0) == rows

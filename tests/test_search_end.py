@@ -30,6 +30,10 @@ int main() {
   show(1, 0, 100, {1, 0}, 1);
   show(4, 0, 4, {1, 4, 2, 7}, 1);      // a full table
   show(3, 0, 100, {1, 4, 2, 0, 1, 0, 0, 0}, 2);
+  std::printf("lists:");
+  for (int rc = 0; rc < 3000; ++rc)
+    if (lists_instead(rc)) std::printf(" %d", rc);
+  std::printf("\n");
 }
 """
 
@@ -49,4 +53,11 @@ def test_a_search_without_a_report_keeps_its_start_only(lines):
 
 
 def test_tables_of_searches_that_ended(lines):
-    assert lines[3:] == ["0 4 | 1 4 2", "0 2 | 1", "0 4 | 1 4 2 7", "0 4 | 1 4 2 | 1"]
+    assert lines[3:7] == ["0 4 | 1 4 2", "0 2 | 1", "0 4 | 1 4 2 7", "0 4 | 1 4 2 | 1"]
+
+
+def test_list_layers_take_over_for_memory_and_residency_only(lines):
+    """UNSUPPORTED, OUT_OF_MEMORY, and cudaErrorCooperativeLaunchTooLarge (720)
+    and cudaErrorNotSupported (801) on the base of CUDA codes; no other error,
+    an illegal address (700) least of all, starts a second search."""
+    assert lines[7] == "lists: 2 3 1720 1801"
