@@ -2250,10 +2250,10 @@ int Graph::run_lists(const mgbfs2_run_limits* limits, mgbfs2_layer_callback cb, 
   no_bitmap = false;
   if (ring) ring->free();
   if (half) half->free();
+  if (coset) coset->free();
   if (coset_ok) {
     // The plan left the bitmap to the run that needs it, in the place of the
     // coset-word buffers.
-    if (coset) coset->free();
     if (int rc = bitmap.ensure((rank_domain() + 63) / 64 * 8)) return rc;
   }
   mgbfs2_status st{};

@@ -173,3 +173,29 @@ def test_a_checkpoint_that_list_layers_cannot_make(tmp_path):
         assert e.layer_table()[0] == want.layer_sizes
         assert sorted(e.frontier_words().tolist()) == words
         assert (e.sample(0), e.sample(1)) == samples
+
+
+def test_list_layers_after_another_plan_hold_no_coset_words():
+    """A handle that ran S12 in coset words (two buffers of 61 MB, a table of 13
+    MB) and is planned again for list layers holds their 60 MB bitmap and small
+    frontiers."""
+    import torch
+    from multigpubfs_b200 import GraphDefinition, native
+    from multigpubfs_b200.engine import NativeGraph
+    graph = GraphDefinition.from_dict(G.permutation_graph(G.lrx_generators(12), list(range(12))))
+
+    def free():
+        native.trim_memory(0)
+        torch.cuda.empty_cache()
+        return torch.cuda.mem_get_info()[0]
+
+    with NativeGraph(graph) as e:
+        e.plan()
+        sizes = e.run().layer_sizes
+    before = free()
+    with NativeGraph(graph) as e:
+        e.plan()
+        assert e.run().layer_sizes == sizes
+        e.plan(dedup="atomic")
+        assert e.run(max_layers=5).layer_sizes == sizes[:5]
+        assert before - free() < 110 << 20
