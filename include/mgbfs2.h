@@ -209,6 +209,13 @@ MGBFS2_API int mgbfs2_plan(mgbfs2_graph* graph, const mgbfs2_plan_request* reque
 MGBFS2_API int mgbfs2_run(mgbfs2_graph* graph, const mgbfs2_run_limits* limits, mgbfs2_layer_callback callback,
                void* user, mgbfs2_status* status);
 
+/* The form in which mgbfs2_run searches under the current plan when it is given
+ * no limits, no callback and no resumed checkpoint (such runs are in LISTS):
+ * frontier lists layer by layer, coset words, unipotent rings or half ranks
+ * (MGBFS2_DEDUP_AUTO above).  MGBFS2_STATE before mgbfs2_plan. */
+enum { MGBFS2_FORM_LISTS = 0, MGBFS2_FORM_COSET = 1, MGBFS2_FORM_RING = 2, MGBFS2_FORM_HALF = 3 };
+MGBFS2_API int mgbfs2_search_form(const mgbfs2_graph* graph, uint32_t* form);
+
 /* layer_sizes / layer_seconds of report.json, generic_run.rs:39. */
 MGBFS2_API int mgbfs2_layer_table(const mgbfs2_graph* graph, uint64_t* sizes, double* seconds, size_t capacity,
                        size_t* count);

@@ -144,20 +144,17 @@ def pilot_depth(layer_sizes: list[int], gens: int, work: int = PILOT_WORK) -> in
     return len(layer_sizes)
 
 
-def runs_coset_layers(graph: GraphDefinition, device: int = 0) -> bool:
-    """Whether the default plan of `graph` runs a whole search in coset-word
-    layers (the Lehmer bitmap of distinct labels, up to 14 symbols and 32
-    generators)."""
-    if graph.action["kind"] != "permutation" or len(graph.start) > 14 or graph.generator_count > 32:
-        return False
+def whole_search(graph: GraphDefinition, device: int = 0) -> bool:
+    """Whether the default plan of `graph` searches without frontier lists
+    (coset words, rings or half ranks) when it is given no limits."""
     from .engine import NativeGraph
     from . import native
     try:
         with NativeGraph(graph, device) as eng:
-            info = eng.plan()
+            eng.plan()
+            return eng.search_form() != "lists"
     except native.NativeError:
         return False
-    return info["visited"] == "bitmap" and info["rank_components"] == 1 and len(set(graph.start)) == len(graph.start)
 
 
 def _run_pilot(graph, plan, device, max_layers, max_seconds, info=None):
@@ -183,7 +180,8 @@ def _trials(graph, plans, device, depth, per_trial, first, started, budget_secon
         r = _run_pilot(graph, plan, device, depth, per_trial)
         want = first.layer_sizes[:depth]
         ok = r is not None and r.layer_sizes[:depth] == want and len(r.layer_sizes) >= len(want)
-        trials.append({"plan": plan, "seconds": r.device_seconds if ok else None})
+        # The wide hash is timed on the host only.
+        trials.append({"plan": plan, "seconds": (r.device_seconds or r.bfs_seconds) if ok else None})
     return trials
 
 
@@ -207,11 +205,12 @@ def choose_profile(graph: GraphDefinition, device: int = 0, *, budget_seconds: f
     started = time.perf_counter()
     plans = candidate_plans(graph)
     per_trial = max(1.0, budget_seconds / (2 * len(plans)))
-    # Coset-word layers run whole searches only, and a prefix of list layers
-    # says nothing about them (S13 LRX: 27 ms, the fastest list layers 144 ms).
-    # Where a whole search is as cheap as a pilot every candidate runs one; the
-    # larger ones keep the default.
-    whole = runs_coset_layers(graph, device)
+    # Coset words, rings and half ranks run whole searches only: a pilot under a
+    # limit would time the list layers that the default does not use (S13 LRX: 27
+    # ms, the fastest list layers 144 ms; 16 positions of four labels: 2.8 and 30
+    # ms).  Where a whole search is as cheap as a pilot every candidate runs one;
+    # the larger ones keep the default.
+    whole = whole_search(graph, device)
     if whole and _state_bound(graph) * graph.generator_count > PILOT_WORK:
         return {"plan": dict(DEFAULT), "source": "size", "trials": []}
     if whole:

@@ -260,3 +260,11 @@ int Graph::half_run(mgbfs2_status* status) {
 }
 
 }  // namespace mgbfs2
+
+extern "C" int mgbfs2_search_form(const mgbfs2_graph* graph, uint32_t* form) {
+  if (!graph || !form) return MGBFS2_INVALID_ARGUMENT;
+  const mgbfs2::Graph& g = *graph->impl;
+  if (!g.planned) return MGBFS2_STATE;
+  *form = g.half_ok ? MGBFS2_FORM_HALF : g.coset_ok ? MGBFS2_FORM_COSET : g.ring_ok ? MGBFS2_FORM_RING : MGBFS2_FORM_LISTS;
+  return MGBFS2_OK;
+}

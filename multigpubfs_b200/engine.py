@@ -151,6 +151,13 @@ class NativeGraph:
         native.check(self.lib.mgbfs2_table_probes(self.handle, C.byref(mean), C.byref(keys)), "mgbfs2_table_probes")
         return float(mean.value), int(keys.value)
 
+    def search_form(self) -> str:
+        """The form of run() without limits or callback under the current plan:
+        "lists", "coset", "ring" or "half" (mgbfs2_search_form)."""
+        form = C.c_uint32()
+        native.check(self.lib.mgbfs2_search_form(self.handle, C.byref(form)), "mgbfs2_search_form")
+        return native.SEARCH_FORMS[form.value]
+
     def checkpoint(self, path):
         """Writes the BFS state after run() (mgbfs2_checkpoint_write)."""
         native.check(self.lib.mgbfs2_checkpoint_write(self.handle, str(path).encode()), "mgbfs2_checkpoint_write")

@@ -21,6 +21,7 @@ VISITED_NAMES = {v: k for k, v in VISITED.items()}
 DEDUP = {"auto": 0, "atomic": 1, "warp": 2, "sort": 3, "bucket": 4, "grouped": 5}
 DEDUP_NAMES = {v: k for k, v in DEDUP.items()}
 PLANNER = {"plain": 0, "learned": 1}
+SEARCH_FORMS = {0: "lists", 1: "coset", 2: "ring", 3: "half"}
 REASONS = {0: "FRONTIER_EXHAUSTED", 1: "DEADLINE", 2: "CANCELLED", 3: "RESOURCE", 4: "PROFILE_LAYER_LIMIT"}
 ERROR_BITS = {1: "FRONTIER_OVERFLOW", 2: "TABLE_FULL", 4: "RANK_RANGE", 8: "BUCKET_OVERFLOW", 16: "WAIT_LIMIT",
               32: "ARENA_OVERFLOW", 64: "BAD_STATE", 128: "BAD_REFERENCE"}
@@ -114,6 +115,7 @@ _SIGNATURES = {
     "mgbfs2_graph_create": (C.c_int, [C.POINTER(GraphDesc), C.c_int, C.POINTER(C.c_void_p), C.c_char_p, C.c_size_t]),
     "mgbfs2_plan": (C.c_int, [C.c_void_p, C.POINTER(PlanRequest), C.POINTER(PlanInfo)]),
     "mgbfs2_run": (C.c_int, [C.c_void_p, C.POINTER(RunLimits), LAYER_CALLBACK, C.c_void_p, C.POINTER(RunStatus)]),
+    "mgbfs2_search_form": (C.c_int, [C.c_void_p, C.POINTER(C.c_uint32)]),
     "mgbfs2_layer_table": (C.c_int, [C.c_void_p, C.POINTER(C.c_uint64), C.POINTER(C.c_double), C.c_size_t,
                                      C.POINTER(C.c_size_t)]),
     "mgbfs2_sample": (C.c_int, [C.c_void_p, C.c_uint32, C.POINTER(C.c_int64), C.c_size_t, C.POINTER(C.c_size_t)]),

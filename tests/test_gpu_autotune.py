@@ -68,3 +68,28 @@ def test_sweep_shape_pilots_stay_exact_then_cache(tmp_path):
         for shape in autotune.SWEEP_SHAPES[1:]:
             sweep.run(**shape)
             assert sweep.layer_tables() == plain, shape
+
+
+@pytest.mark.parametrize("start", [[0, 1, 2, 3] * 4, [0, 1, 2, 3, 4] * 2 + [0, 1, 2, 3], [0, 1] * 14])
+def test_repeated_labels_keep_their_half_ranks(tmp_path, monkeypatch, start):
+    """63 M states (past a pilot's work), 34 M, and 40 M of 28 positions: the
+    default is timed as it runs, or not at all, and is what run_graph takes."""
+    from multigpubfs_b200 import GraphDefinition, autotune
+    from multigpubfs_b200.engine import NativeGraph
+    from multigpubfs_b200.launch import run_graph
+    g = GraphDefinition.permutation(G.lrx_generators(len(start)), start)
+    got = autotune.choose_profile(g, 0, cache=tmp_path / "tune.json")
+    assert got["plan"] == autotune.DEFAULT
+    with NativeGraph(g) as e:
+        e.plan(**got["plan"])
+        assert e.search_form() == "half"
+        sizes = e.run().layer_sizes
+    if len(start) == 16:
+        assert got["source"] == "size"
+    else:
+        cands = autotune.candidate_plans(g)
+        seconds = [t["seconds"] for t in got["trials"][:len(cands)]]
+        assert got["source"] == "pilot" and all(seconds[0] < s for s in seconds[1:] if s is not None)
+    monkeypatch.setenv("MGBFS2_AUTOTUNE_CACHE", str(tmp_path / "tune.json"))
+    report = run_graph(g, tmp_path / "out", autotune=True)
+    assert report["autotune"]["plan"] == autotune.DEFAULT and report["layer_sizes"] == sizes
