@@ -25,6 +25,7 @@
 #include "bucket_kernels.cuh"
 #include "coset.h"
 #include "engine.h"
+#include "group.h"
 #include "grouped_kernels.cuh"
 #include "half.h"
 #include "packed_kernels.cuh"
@@ -1323,11 +1324,20 @@ int Graph::make_plan(const mgbfs2_plan_request* req, mgbfs2_plan_info* out) {
   // layers (coset.h) where their buffers fit: nothing asked for that only the
   // list layers have (a dedup, a frontier capacity, shapes, the host loop), and
   // no caller's bound below the rank domain that a layer might have to break.
+  // A layer looks at every row's flags, and the buffers are cleared whole: at 13
+  // and 14 symbols a group other than A_n and S_n, which has less than 1/400 of
+  // the states, is searched faster in lists (C13, 7 layers: 0.68 ms a call
+  // against 0.92; 156 states of AGL(1,13): 0.79, 1.14; S14, 645,120 states of S2
+  // wr S7: 3.1, 29.7; 50.8 M of S7 wr S2: 7.3, 43.7; A13: 105, 14.7).  At 12 lists
+  // win some repeated calls (82,944 states of S4 wr S3: 0.61, 0.93; C12: 0.44,
+  // 0.36) and lose first ones, where they map 7.4 GB for a bound of 12! states
+  // (S4 wr S3: 2.9, 2.0; C12: 22, 1.4): coset words for all.
   const CosetJob job{elements, gens, perms.data(), inverse_closed};
   coset_ok = visited == MGBFS2_VISITED_BITMAP && r.dedup == MGBFS2_DEDUP_AUTO && lehmer && !use_product &&
              !host_loop_only && !r.capacity && !r.shards && !r.group_chunk && !r.blocks_per_sm &&
              !r.parents_per_thread && !r.route_chunk && !r.bucket_min_work && !r.bucket_margin &&
              (!orbit_bound || orbit_bound >= rank_total) && coset_supported(elements, gens) &&
+             (!coset_wide(elements) || group_is_giant(perms.data(), elements, gens)) &&
              coset_job_bytes(job, kWholeDepth) + coset_fixed_bytes(kWholeDepth) <= budget / 2;
   // Likewise invertible 2x2 matrices over a prime field in unipotent-ring
   // layers (ring.h), from the layer on where they overtake the list layers.  A

@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "../../include/mgbfs2.h"
+#include "group.h"
 
 namespace mgbfs2 {
 namespace {
@@ -416,6 +417,18 @@ int graph_statics(const uint32_t* perms, uint32_t n, uint32_t k, const uint32_t*
 }
 
 }  // namespace
+
+bool group_is_giant(const uint32_t* permutations, uint32_t n, uint32_t generators) {
+  if (n > kMaxPoints) return false;
+  std::vector<Perm> gens;
+  for (uint32_t g = 0; g < generators; ++g) {
+    Perm p = identity();
+    for (uint32_t i = 0; i < n; ++i) p[i] = static_cast<uint8_t>(permutations[static_cast<size_t>(g) * n + i]);
+    if (!is_identity(p)) gens.push_back(p);
+  }
+  return contains_alternating(gens, n);
+}
+
 }  // namespace mgbfs2
 
 extern "C" int mgbfs2_group_order(const uint32_t* permutations, uint32_t n, uint32_t generators, uint64_t* order) {

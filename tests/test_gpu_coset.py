@@ -199,3 +199,41 @@ def test_list_layers_after_another_plan_hold_no_coset_words():
         e.plan(dedup="atomic")
         assert e.run(max_layers=5).layer_sizes == sizes[:5]
         assert before - free() < 110 << 20
+
+
+def _wreath(k, blocks):
+    """S_k wr S_blocks on k * blocks points: two generators of one block, two of
+    the blocks."""
+    n = k * blocks
+    return [list(range(1, k)) + [0] + list(range(k, n)), [1, 0] + list(range(2, n)),
+            [(i + k) % n for i in range(n)], list(range(k, 2 * k)) + list(range(k)) + list(range(2 * k, n))]
+
+
+@pytest.mark.parametrize("name,form", [("C12", "coset"), ("C13", "lists"), ("AGL(1,13)", "lists"), ("S2 wr S7", "lists"),
+                                       ("S7 wr S2", "lists"), ("A13", "coset"), ("LRX13", "coset"), ("S13", "coset"),
+                                       ("S14", "coset")])
+def test_small_orbits_of_wide_words_are_searched_in_lists(name, form):
+    """At 13 and 14 symbols a group other than A_n and S_n keeps list layers;
+    its table is that of the oracle, or of its bound."""
+    from multigpubfs_b200 import GraphDefinition
+    from multigpubfs_b200.engine import NativeGraph
+    rng = random.Random(14)
+    gens = {"C12": lambda: _closed([list(range(1, 12)) + [0]]), "C13": lambda: _closed([list(range(1, 13)) + [0]]),
+            "AGL(1,13)": lambda: [[(i + 1) % 13 for i in range(13)], [2 * i % 13 for i in range(13)]],
+            "S2 wr S7": lambda: _closed(_wreath(2, 7)), "S7 wr S2": lambda: _wreath(7, 2),
+            "A13": lambda: [list(range(1, 13)) + [0], [1, 2, 0] + list(range(3, 13))],
+            "LRX13": lambda: G.lrx_generators(13),
+            "S13": lambda: [rng.sample(range(13), 13) for _ in range(3)],
+            "S14": lambda: _closed([rng.sample(range(14), 14) for _ in range(2)])}[name]()
+    graph = G.permutation_graph(gens, rng.sample(range(len(gens[0])), len(gens[0])))
+    with NativeGraph(GraphDefinition.from_dict(graph)) as e:
+        e.plan()
+        assert e.search_form() == form
+        if name in ("A13", "LRX13", "S13", "S14"):
+            return
+        r = e.run()
+        assert r.complete and e.search_form() == form
+        if name == "S7 wr S2":
+            assert sum(r.layer_sizes) == 2 * 5040 ** 2
+        else:
+            assert r.layer_sizes == P.packed_bfs(gens, graph["start"], max_states=1 << 20)[0]
