@@ -1112,7 +1112,7 @@ int mgbfs2_batch_run(mgbfs2_batch* batch, const mgbfs2_batch_options* options, m
     for (uint32_t i : wave) coset = coset && coset_supported(b->inst[i].n, b->inst[i].gens);
     if (coset) {
       std::vector<uint32_t> same;
-      uint64_t need = coset_fixed_bytes(max_depth);
+      std::vector<CosetJob> jobs;
       for (uint32_t i : wave) {
         const auto& in = b->inst[i];
         if (coset_wide(in.n) != coset_wide(b->inst[wave[0]].n)) {
@@ -1120,9 +1120,9 @@ int mgbfs2_batch_run(mgbfs2_batch* batch, const mgbfs2_batch_options* options, m
           continue;
         }
         same.push_back(i);
-        need += coset_job_bytes(CosetJob{in.n, in.gens, nullptr, in.inverse_closed}, max_depth);
+        jobs.push_back(CosetJob{in.n, in.gens, nullptr, in.inverse_closed});
       }
-      if (need <= budget) wave.swap(same);
+      if (coset_wave_bytes(jobs, max_depth) <= budget) wave.swap(same);
       else coset = false;
       if (!coset) later.resize(later.size() - (wave.size() - same.size()));
     }

@@ -160,13 +160,6 @@ __host__ __device__ __forceinline__ uint32_t row_rank(uint32_t m, const uint8_t*
   return row;
 }
 
-__host__ __device__ __forceinline__ uint32_t rows_of(uint32_t m) {
-  const uint32_t outer = m - kSlots;
-  uint32_t r = outer & 1 ? 8 : 1;
-  for (uint32_t t = 0; t < outer / 2; ++t) r *= (m - 2 * t) * (m - 2 * t - 1) / 2;
-  return r;
-}
-
 // Slots of a node's inner labels, four bits a label, each pair's lower slot
 // first.
 constexpr uint32_t packed_slots(uint32_t x) {
@@ -1074,25 +1067,13 @@ __global__ void __launch_bounds__(kCosetBlock) coset_small_collect(SmallParams p
 
 size_t al256(size_t x) { return (x + 255) / 256 * 256; }
 
-uint32_t embedded(uint32_t n) { return std::max(n, kSlots); }
-
-size_t table_bytes() { return static_cast<size_t>(kSlotPerms) * kCosetStride * sizeof(uint32_t); }
+static_assert(kSlots == kCosetInner && kSlotPerms == kCosetInnerPerms && sizeof(CosetInst) <= kCosetInstBytes,
+              "the sizes coset_bytes.h counts with");
 
 }  // namespace
 
 bool coset_supported(uint32_t n, uint32_t gens) {
   return n >= 2 && n <= kCosetMaxDegree && gens >= 1 && gens <= kCosetMaxGens;
-}
-
-uint64_t coset_job_bytes(const CosetJob& job, uint32_t max_depth) {
-  const uint32_t rows = rows_of(embedded(job.n));
-  const uint64_t word = coset_wide(job.n) ? 8 : 4, buffers = job.inverse_closed ? 2 : 3;
-  return rows * (buffers * kCosetStride * word + 20 + 8ull * job.gens) + sizeof(CosetInst) + 4 + 16ull * job.gens +
-         8ull * (max_depth + 2);
-}
-
-uint64_t coset_fixed_bytes(uint32_t max_depth) {
-  return table_bytes() + kSlotPerms + 16ull * kCosetSmall + 20ull * (max_depth + 2) + 32 * 256;
 }
 
 // Layer tables (count x end.columns sizes) and step times.
@@ -1112,7 +1093,7 @@ static int coset_small(const CosetJob& job, uint32_t max_depth, uint32_t units, 
                        CosetMemory* memory, CosetResult* out, DeviceBuffer* collect, uint64_t start_word) {
   SmallParams p{};
   p.n = job.n;
-  p.m = embedded(job.n);
+  p.m = coset_symbols(job.n);
   p.gens = job.gens;
   p.units = units;
   p.inverse_closed = job.inverse_closed;
@@ -1203,7 +1184,7 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   uint64_t units = 0;
   for (const CosetJob& j : jobs) {
     if (!coset_supported(j.n, j.gens) || coset_wide(j.n) != wide || !j.perms) return MGBFS2_INVALID_ARGUMENT;
-    units += static_cast<uint64_t>(rows_of(embedded(j.n))) * kCosetParts;
+    units += static_cast<uint64_t>(coset_rows(j.n)) * kCosetParts;
   }
   const uint64_t warps = static_cast<uint64_t>(per_sm) * sm_count * (threads / 32);
   uint32_t per_item = kMaxUnits;
@@ -1224,14 +1205,14 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   std::vector<CosetInst> inst(count);
   std::vector<uint32_t> prefix(count + 1, 0);
   std::vector<uint8_t> perms;
-  unsigned long long rows = 0, descs = 0, visited_rows = 0;
+  unsigned long long rows = 0, descs = 0;
   bool walks = false;
   for (uint32_t i = 0; i < count; ++i) {
     const CosetJob& j = jobs[i];
     CosetInst& c = inst[i];
-    c.m = embedded(j.n);
+    c.m = coset_symbols(j.n);
     c.gens = j.gens;
-    c.rows = rows_of(c.m);
+    c.rows = coset_rows(j.n);
     c.inverse_closed = j.inverse_closed;
     c.same_layer = 0;
     c.perm_off = static_cast<uint32_t>(perms.size());
@@ -1263,7 +1244,6 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
     walks |= c.walk != kNoWalk;
     rows += c.rows;
     descs += static_cast<unsigned long long>(c.rows) * c.gens;
-    if (!j.inverse_closed) visited_rows = rows;
     prefix[i + 1] = prefix[i] + (c.rows * kCosetParts + per_item - 1) / per_item;
   }
   // Arena: uploaded block | cleared block (tables of the loop, flags, buffers) | tables.
@@ -1280,12 +1260,12 @@ int coset_wave(const std::vector<CosetJob>& jobs, uint32_t max_depth, int sm_cou
   const size_t o_ctl = take(sizeof(CosetCtl)), o_used = take(kSlotPerms);
   const size_t o_flags0 = take(8 * rows), o_flags1 = take(8 * rows);
   const size_t word_bytes[3] = {rows * kCosetStride * word, rows * kCosetStride * word,
-                                visited_rows * kCosetStride * word};
+                                coset_visited_rows(jobs) * kCosetStride * word};
   const bool own = word_bytes[0] >= kCosetOwnWords;
   size_t o_words[3];
   for (int k = 0; k < 3; ++k) o_words[k] = take(own ? 0 : word_bytes[k]);
   const size_t cleared = off;
-  const size_t o_stamps = take(8ull * stride), o_small = take(16ull * kCosetSmall), o_table = take(table_bytes());
+  const size_t o_stamps = take(8ull * stride), o_small = take(16ull * kCosetSmall), o_table = take(coset_table_bytes());
   const size_t o_desc = take(8 * descs);
   const uint64_t order_blocks = (rows + kOrderBlock - 1) / kOrderBlock;
   const size_t o_order = take(wide ? 4 * rows : 0), o_order_sums = take(wide ? 4 * order_blocks : 0);

@@ -36,6 +36,7 @@
 #include <vector>
 
 #include "../../include/mgbfs2.h"
+#include "coset_bytes.h"
 #include "engine.h"
 
 namespace mgbfs2 {
@@ -43,16 +44,7 @@ namespace mgbfs2 {
 constexpr uint32_t kCosetMaxDegree = 14;
 constexpr uint32_t kCosetMaxGens = 32;
 constexpr uint32_t kCosetNodes = 630;    // nodes of a row
-constexpr uint32_t kCosetStride = 640;   // words of a row in memory: 5 parts of 128
 constexpr uint32_t kCosetParts = 5;
-constexpr uint32_t kCosetSmall = 1000;   // layers of fewer states are kept for samples
-
-// One search of a wave.
-struct CosetJob {
-  uint32_t n = 0, gens = 0;
-  const uint32_t* perms = nullptr;  // gens x n, child[i] = state[g[i]]
-  bool inverse_closed = false;
-};
 
 // Device memory of a wave.  Word buffers from kCosetOwnWords bytes up are
 // allocations of their own: given back to the device cache they have the size
@@ -95,11 +87,6 @@ struct CosetResult {
 };
 
 bool coset_supported(uint32_t n, uint32_t gens);
-// 64-bit words: jobs of one wave must agree.
-inline bool coset_wide(uint32_t n) { return n >= 13; }
-// Device bytes of a job's buffers and tables in a wave.
-uint64_t coset_job_bytes(const CosetJob& job, uint32_t max_depth);
-uint64_t coset_fixed_bytes(uint32_t max_depth);
 
 // Runs every job to the end (or max_depth layers) in one cooperative launch
 // on `stream`, in `memory` (grown as needed).  With `collect`, the wave holds

@@ -1338,7 +1338,7 @@ int Graph::make_plan(const mgbfs2_plan_request* req, mgbfs2_plan_info* out) {
              !r.parents_per_thread && !r.route_chunk && !r.bucket_min_work && !r.bucket_margin &&
              (!orbit_bound || orbit_bound >= rank_total) && coset_supported(elements, gens) &&
              (!coset_wide(elements) || group_is_giant(perms.data(), elements, gens)) &&
-             coset_job_bytes(job, kWholeDepth) + coset_fixed_bytes(kWholeDepth) <= budget / 2;
+             coset_wave_bytes({job}, kWholeDepth) <= budget / 2;
   // Likewise invertible 2x2 matrices over a prime field in unipotent-ring
   // layers (ring.h), from the layer on where they overtake the list layers.  A
   // singular start reaches fewer than p^2 states.
