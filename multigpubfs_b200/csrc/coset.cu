@@ -54,7 +54,7 @@ struct CosetParams {
   const uint32_t* item_prefix;  // count + 1: exclusive prefix of the jobs' work items
   const uint8_t* perms;
   uint32_t count, units;        // jobs; units per item (a power of two)
-  uint32_t chunk, spare;        // 64-bit words: items of a block's chunk
+  uint32_t chunk;               // 64-bit words: items of a block's chunk
   uint32_t stride, max_steps;   // layer-table columns; last step that may run
   unsigned long long* counts;   // count x stride layer sizes
   uint32_t* active;             // stride: layer d of any job is not empty
@@ -73,7 +73,7 @@ struct CosetParams {
   CosetReport* report;          // wave of one job: written at the end, else null
   unsigned long long* front;    // with report: states of the deepest layer, as far as front_cap
   unsigned long long front_cap, start;  // start: the start's codes, 4 bits each
-  uint32_t n, pad;
+  uint32_t n;                   // with report: symbols of the job
   unsigned long long descs;     // total descriptors
   CosetCtl* ctl;
 };
