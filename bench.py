@@ -77,7 +77,8 @@ def coxeter(n):
 
 WORKLOADS = {
     "s13-lrx": dict(n=13, gens=lrx(13), visited="bitmap", dedup="auto",
-                    desc="S13 LRX full BFS (L, R, X from identity; 6,227,020,800 states), exact Lehmer-rank bitmap"),
+                    desc="S13 LRX full BFS (L, R, X from identity; 6,227,020,800 states), exact bitmap of the "
+                         "rank domain"),
     "s14-lrx": dict(n=14, gens=lrx(14), visited="bitmap", dedup="auto",
                     desc="S14 LRX full BFS (87,178,291,200 states, 4.6e9 in the peak layer), exact bitmap of the "
                          "rank domain"),
@@ -334,11 +335,11 @@ def roofline(b_alg, seconds, kernel, traffic=None, traffic_source=None, **extra)
     return out
 
 
-def whole_search_words(workload, plan):
-    """(words, states per word, bytes per word, kind, kernel) of a search that
-    the default plan runs without frontier lists, None for list layers: coset
-    words of distinct labels, bit rings of 2x2 matrices over a prime field."""
-    if plan["visited"] != "bitmap":
+def whole_search_words(workload, form):
+    """(words, states per word, bytes per word, kind, kernel) of a search in
+    `form` (NativeGraph.search_form), None for list layers: coset words of
+    distinct labels, bit rings of 2x2 matrices over a prime field."""
+    if form not in ("coset", "ring"):
         return None
     if "matrix_p" in workload:
         p = workload["matrix_p"]
@@ -627,6 +628,7 @@ def bench_single(args, rank, world, local):
     # ---- value: resident engine, K whole BFS runs ------------------------------------
     eng = NativeGraph(graph, local)
     plan = eng.plan(visited=visited, dedup=dedup, host_loop=args.host_loop)
+    form = eng.search_form()
     for _ in range(args.warmup):
         r = eng.run()
         assert table_ok(r.layer_sizes), "layer table mismatch in warm-up"
@@ -691,7 +693,7 @@ def bench_single(args, rank, world, local):
         dist.all_reduce(e2e_t, op=dist.ReduceOp.MAX)
 
     if rank == 0:
-        words = None if dedup != "auto" or args.host_loop else whole_search_words(w, plan)
+        words = whole_search_words(w, form)
         b_alg = word_bytes(results[0].layer_sizes, *words[:4]) if words else int(16 * states + 32 * succ * probes)
         traffic, source = None, None
         prof = ROOT / "profiles" / f"traffic_{args.workload}.json"
@@ -722,6 +724,7 @@ def bench_single(args, rank, world, local):
                        "planner": plan["planner"], "parallelism": f"replicas{world}" + (
                            " (each GPU runs the whole BFS; the BFS itself is not split)" if world > 1 else ""),
                        "states_per_bfs": states, "successors_per_bfs": succ, "visited_tests_per_bfs": tests,
+                       **({"visited_tests": "what list layers would test; words are pulled whole"} if words else {}),
                        "l2": ("working set %s than L2 (%%s)" % ("smaller" if words and 2 * words[0] * words[2] < 126 << 20
                                                                 else "larger")) % (
                            "two word buffers of %d MB" % (words[0] * words[2] >> 20) if words else
