@@ -65,10 +65,12 @@ enum { MGBFS2_VISITED_AUTO = 0, MGBFS2_VISITED_BITMAP = 1, MGBFS2_VISITED_HASH =
  * AUTO names one of these for layers over frontier lists (runs with limits, a
  * callback or a resumed checkpoint, plans that set a capacity, a shape or the
  * host loop) and runs a whole search without frontier lists where it can:
- * distinct labels up to degree 14 and 32 generators in coset-word layers,
- * inverse-closed invertible 2x2 matrices over primes 17..257 in unipotent-ring layers, up to
- * six repeated labels in half-rank layers (csrc/coset.h, ring.h, half.h).  The
- * results are the same. */
+ * distinct labels up to degree 14 and 32 generators in coset-word layers (at 13
+ * and 14 where the generators make A_n or S_n), inverse-closed invertible 2x2
+ * matrices over primes 17..257 in unipotent-ring layers, up to six repeated
+ * labels and 512 displacement terms in half-rank layers (csrc/coset.h, ring.h,
+ * half.h; mgbfs2_search_form says which).  The results are the same, and a run
+ * whose buffers or grid do not fit goes on in list layers. */
 enum { MGBFS2_DEDUP_AUTO = 0, MGBFS2_DEDUP_ATOMIC = 1, MGBFS2_DEDUP_WARP = 2, MGBFS2_DEDUP_SORT = 3,
        MGBFS2_DEDUP_BUCKET = 4, MGBFS2_DEDUP_GROUPED = 5 };
 enum { MGBFS2_PLANNER_PLAIN = 0, MGBFS2_PLANNER_LEARNED = 1 };
@@ -230,7 +232,10 @@ MGBFS2_API int mgbfs2_sample(mgbfs2_graph* graph, uint32_t which, int64_t* out, 
  * limit, deadline or cancel, or complete): the layer table, the visited
  * structure (bitmap or all-visited hash), the deepest layer and the small-layer
  * samples, written to `path`.  Bitmap and all-visited hash plans of one-word
- * states (three-bank histories and wide states: MGBFS2_UNSUPPORTED). */
+ * states (three-bank histories and wide states: MGBFS2_UNSUPPORTED).  After a
+ * search in coset words or rings list layers run once more for the bitmap; where
+ * they end short of the search's table (MGBFS2_CAPACITY, MGBFS2_OUT_OF_MEMORY)
+ * nothing is written and the handle keeps the search's results. */
 MGBFS2_API int mgbfs2_checkpoint_write(mgbfs2_graph* graph, const char* path);
 
 /* Loads a checkpoint into a handle planned for the same graph and visited

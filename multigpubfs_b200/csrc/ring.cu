@@ -203,7 +203,9 @@ __device__ void ring_report(const RingParams& r, uint32_t d, bool exhausted) {
 
 // A layer is a pass over the rings of the determinants that it can hold, a
 // warp per 32 rings: per generator one coalesced move, one ring of 32 bytes and
-// about 65 instructions, half of them the rotation's, which bound it.  GL(2,211),
+// its rotation, most of the instructions.  No unit is full (integer pipe 48 % of
+// its rate, issue slots 43 %, DRAM 0.6 TB/s): the warps wait for the ring loads,
+// whose addresses hang on the moves, and at the barrier behind uneven layers.  GL(2,211),
 // 111 layers, whole call: 4.8 ms, 30 to 60 us a layer; rings of the 210 scalar
 // multiples, which mix all determinants (520 us a layer): 58.8 ms; list layers:
 // 271 ms.  GL(2,257): 9.4 ms.

@@ -18,7 +18,7 @@ def _search(graph, **plan):
         return r, e.sample(0, 1000), e.sample(1, 1000), sorted(e.frontier_words().tolist())
 
 
-# 13 and 263 are past the rings' primes; 101 and 103 lie on the two sides of
+# 13 is below the rings' primes; 101 and 103 lie on the two sides of
 # the node count from which list layers go first.
 @pytest.mark.parametrize("p", [13, 17, 31, 37, 61, 67, 101, 103, 127, 131])
 @pytest.mark.parametrize("start", [[1, 0, 0, 1], [2, 5, 3, 1], [0, 0, 4, 7], [0, 3, 0, 0]])
