@@ -162,8 +162,14 @@ def test_a_checkpoint_that_list_layers_cannot_make(tmp_path):
         assert max(want.layer_sizes) > 6 << 20  # more than (96 MB - the bitmap) / 16 bytes
         native.trim_memory(0)
         torch.cuda.empty_cache()
-        free, _ = torch.cuda.mem_get_info()
-        e.plan(reserve_bytes=free - (96 << 20))
+        # The plan's free memory may be some seconds old: its own capacity (16
+        # bytes a state beside the bitmap) says what budget a reserve leaves.
+        reserve = torch.cuda.mem_get_info()[0] - (300 << 20)
+        info = e.plan(reserve_bytes=reserve)
+        assert info["capacity"] < info["state_bound"]
+        reserve += 16 * info["capacity"] + info["bitmap_bits"] // 8 - (96 << 20)
+        info = e.plan(reserve_bytes=reserve)
+        assert 5 << 20 < info["capacity"] < 6 << 20 and e.search_form() == "coset"
         r = e.run()
         assert r.complete and r.layer_sizes == want.layer_sizes
         path = tmp_path / "refused.bin"
